@@ -1,4 +1,5 @@
-"""ctypes binding of ``libllnvfp4.so``.  There is no fallback: a missing library is an error."""
+"""Loading of ``libllnvfp4.so`` (ctypes: the whole C ABI) and of ``_native.so`` (the compiled binding the operations of
+``ops.py`` call).  There is no fallback: a missing library is an error."""
 from __future__ import annotations
 
 import ctypes as C
@@ -102,6 +103,23 @@ def lib() -> C.CDLL:
             getattr(l, name)
         _lib = l
     return _lib
+
+
+_native = None
+
+
+def native():
+    """The compiled binding (``csrc/binding.cpp``): one function per operation of ``ops.py``."""
+    global _native
+    if _native is None:
+        lib()
+        try:
+            from . import _native as mod
+        except ImportError as exc:
+            raise LibraryMissing("longlive_b200/_native.so is missing or was built for another PyTorch: build it with "
+                                 f"`python -m longlive_b200.build` ({exc})") from exc
+        _native = mod
+    return _native
 
 
 _ready_devices: set = set()

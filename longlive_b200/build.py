@@ -1,8 +1,10 @@
-"""In-tree build of ``libllnvfp4.so`` (the C-ABI library) with nvcc for sm_100a.
+"""In-tree build of ``libllnvfp4.so`` (the C-ABI library) with nvcc for sm_100a, and of ``_native.so``
+(its Python binding) with g++ against the installed PyTorch.
 
 ``python -m longlive_b200.build`` compiles every ``csrc/*.cu`` into one object each (in
-parallel) and links them into ``longlive_b200/libllnvfp4.so``.  Objects are rebuilt only when a
-source or header is newer.  nvcc cross-compiles without a GPU.
+parallel) and links them into ``longlive_b200/libllnvfp4.so``, then ``csrc/binding.cpp`` into
+``longlive_b200/_native.so``.  Objects are rebuilt only when a source or header is newer.  nvcc
+cross-compiles without a GPU.
 """
 from __future__ import annotations
 
@@ -17,6 +19,7 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(PKG, "build")
 LIB = os.path.join(PKG, "libllnvfp4.so")
+NATIVE = os.path.join(PKG, "_native.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -33,6 +36,27 @@ def _nvcc() -> str:
 
 def _newest(paths) -> float:
     return max(os.path.getmtime(p) for p in paths)
+
+
+def _build_binding(verbose: bool, force: bool) -> None:
+    src = os.path.join(CSRC, "binding.cpp")
+    newest = _newest([src, os.path.join(PKG, "..", "include", "llnvfp4.h")])
+    if not force and os.path.exists(NATIVE) and os.path.getmtime(NATIVE) >= newest:
+        return
+    import sysconfig
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+    cuda_home = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    inc = [*include_paths(), os.path.join(cuda_home, "include"), sysconfig.get_paths()["include"]]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_native",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-isystem{p}" for p in inc), src, "-o", NATIVE,
+           f"-L{PKG}", "-lllnvfp4", "-Wl,-rpath,$ORIGIN", *(f"-L{p}" for p in library_paths()), "-lc10", "-lc10_cuda", "-ltorch_cpu",
+           "-ltorch", "-ltorch_python"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or r.returncode != 0:
+        sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+    if r.returncode != 0:
+        raise RuntimeError("build of _native.so failed")
 
 
 def build(verbose: bool = False, force: bool = False) -> str:
@@ -68,6 +92,7 @@ def build(verbose: bool = False, force: bool = False) -> str:
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link of libllnvfp4.so failed")
+    _build_binding(verbose, force)
     return LIB
 
 

@@ -12,9 +12,15 @@ from typing import Any, Callable, ClassVar
 import torch
 import torch.nn as nn
 
+from . import _lib
 from .enums import DataType, MatmulBackend, QuantizeBackend, RoundStyle, ScaleRule
 from .matmul import fp4_matmul
 from .quantize import QuantizationConfig, QuantizedTensor, quantize_to_fp4
+
+
+_ACTIVATIONS = (torch.bfloat16, torch.float16)
+_QUANTIZE_BACKENDS = (None, QuantizeBackend.cuda)
+_MATMUL_BACKENDS = (None, MatmulBackend.cutlass)
 
 
 def _enum(cls, v):
@@ -190,6 +196,13 @@ class FourOverSixLinear(nn.Linear):
         w = self.quantized_weight()
         if not isinstance(w, QuantizedTensor):
             w = quantize_to_fp4(w.data, self.config.get_weight_config())
+        cfg = self.config
+        if (input.is_cuda and input.dtype in _ACTIVATIONS and cfg.dtype is DataType.nvfp4 and cfg.output_dtype is DataType.bfloat16
+                and cfg.quantize_backend in _QUANTIZE_BACKENDS and cfg.matmul_backend in _MATMUL_BACKENDS
+                and input.shape[-1] == w.original_shape[1] == w.padded_shape[1] and w.padded_shape[1] % 256 == 0 and input.numel()):
+            # the same three steps as below in one native call: at few tokens the module call is bound by the host
+            return _lib.native().linear_nvfp4(input, cfg.activation_scale_rule.cuda_id(), w.values, w.scale_factors, w.amax,
+                                              w.scale_rule.cuda_id(), w.original_shape[0], w.padded_shape[0], w.padded_shape[1], self.bias)
         x2d = input.reshape(-1, input.shape[-1])
         xq = quantize_to_fp4(x2d, self.config.get_activation_config())
         out = fp4_matmul(xq, w, backend=self.config.matmul_backend, out_dtype=self.config.output_dtype, bias=self.bias)

@@ -22,7 +22,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .ops import _check, _require_cuda, _stream
+from .ops import _require_cuda
 
 
 def _lam(sigma: torch.Tensor) -> torch.Tensor:
@@ -92,6 +92,7 @@ class FlowUniPCMultistepScheduler:
         self.sigma_max = self.sigmas[0].item()
         self.num_inference_steps = None
         self._coef_cache: dict = {}
+        self._grids: dict = {}
         self._buffers = None
         self._reset()
 
@@ -108,21 +109,29 @@ class FlowUniPCMultistepScheduler:
 
     def set_timesteps(self, num_inference_steps: int, device=None, sigmas=None, mu=None, shift: float | None = None) -> None:
         """Sigma grid and integer timesteps of a run (fm_solvers_unipc.py:162-229); clears the step state."""
-        if sigmas is None:
-            sigmas = np.linspace(self.sigma_max, self.sigma_min, num_inference_steps + 1).copy()[:-1]
-        else:
-            sigmas = np.asarray(sigmas, dtype=np.float64)
         if shift is None:
             shift = self.shift
-        sigmas = shift * sigmas / (1 + (shift - 1) * sigmas)
-        timesteps = sigmas * self.num_train_timesteps
-        new_sigmas = torch.from_numpy(np.concatenate([sigmas, [0]]).astype(np.float32))
+        # the grid of (steps, shift) is a host table of a few numbers; a video sets the same one for every chunk
+        key = (num_inference_steps, shift) if sigmas is None else None
+        grid = self._grids.get(key) if key is not None else None
+        if grid is None:
+            if sigmas is None:
+                sigmas = np.linspace(self.sigma_max, self.sigma_min, num_inference_steps + 1).copy()[:-1]
+            else:
+                sigmas = np.asarray(sigmas, dtype=np.float64)
+            sigmas = shift * sigmas / (1 + (shift - 1) * sigmas)
+            host = (sigmas * self.num_train_timesteps).astype(np.int64)
+            grid = (torch.from_numpy(np.concatenate([sigmas, [0]]).astype(np.float32)), torch.from_numpy(host), host.tolist())
+            if key is not None:
+                if len(self._grids) >= 64:
+                    self._grids.clear()
+                self._grids[key] = grid
+        new_sigmas, timesteps, self._timesteps_host = grid
         if self.num_inference_steps is None or not torch.equal(new_sigmas, self.sigmas):
             self._coef_cache = {}                             # same grid as the last run: its coefficients stand
-        self.sigmas = new_sigmas
-        self.timesteps = torch.from_numpy(timesteps).to(device=device, dtype=torch.int64)
-        self._timesteps_host = [int(t) for t in timesteps.astype(np.int64)]
-        self.num_inference_steps = len(timesteps)
+        self.sigmas = new_sigmas.clone()
+        self.timesteps = timesteps.to(device=device, copy=True)
+        self.num_inference_steps = len(self._timesteps_host)
         self._reset()
 
     def _orders(self, k: int) -> tuple[int, int]:
@@ -187,12 +196,7 @@ class FlowUniPCMultistepScheduler:
         need_older = coef.use_corrector and coef.corrector_order == 2
         if (need_prev and self._hist < 1) or (need_older and self._hist < 2):
             raise RuntimeError("step() was entered in the middle of a schedule without the earlier steps' history")
-        v, x = model_output.contiguous(), sample.contiguous()
-        out = torch.empty_like(x)
-        with torch.cuda.device(x.device):
-            _check(_lib.lib().llnv_unipc_step(v.data_ptr(), x.data_ptr(), prev.data_ptr(), older.data_ptr(), last.data_ptr(),
-                                              older.data_ptr(), last.data_ptr(), out.data_ptr(), x.numel(),
-                                              0 if x.dtype == torch.bfloat16 else 1, C.byref(coef), _stream(x)))
+        out = _lib.native().unipc_step(model_output, sample, prev, older, last, C.addressof(coef))
         self._buffers[1][0], self._buffers[1][1] = prev, older   # the new x0 went where the oldest one was
         self._hist = min(2, self._hist + 1)
         self._have_last = True
