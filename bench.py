@@ -445,7 +445,7 @@ def attention_roofline(dev, rank, world, peaks, iters=8):
     peak = peaks["bf16_tflops"]
     return {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
             "traffic": (lambda t: None if t is None else t * heads / 24.0)(dram_traffic("attention_kernel<fused>", "2640x4x2640x24")),
-            "traffic_case": "ncu capture at 24 heads (profiles/dram_traffic.md), scaled by heads / 24", "kernel": "attention_kernel<true> (NVFP4 K/V decoded in the load stage)",
+            "traffic_case": "ncu capture at 24 heads (profiles/dram_traffic.md), scaled by heads / 24", "kernel": "attention_kernel behind one launch that expands the NVFP4 blocks to bf16",
             "shape": f"{t} queries x {(blocks + 1) * t} keys x {heads} heads", "avg_launch_us": ms * 1e3, "launches_timed": iters,
             "algorithmic_flops_per_launch": fl,
             "peak_note": f"{peaks['source']} dense bf16 burst peak (cuBLAS GEMM); the kernel's MMAs are bf16 (kind::f16)"}
@@ -626,7 +626,7 @@ def run_gpu_arm(args):
                                "peak_note": f"GEMM flops at 4 x {peaks['source']} sustained bf16 peak ({peaks['bf16_tflops_sustained']} TFLOP/s), "
                                             f"attention flops at that peak, divided over {world} GPU(s)"},
             "memory": {"kv_cache_bytes_per_rank": kv_bytes, "current_chunk_kv_bytes_per_rank": cur_bytes,
-                       "note": "no bf16 copy of the cache exists: the attention kernel decodes the NVFP4 blocks in its load stage"},
+                       "note": "the cached window of one layer at a time is expanded to bf16 in a workspace all layers share"},
             "wall_s_timed_region": wall,
         }
         if sp_parity is not None:

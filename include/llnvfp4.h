@@ -301,15 +301,14 @@ int llnv_attention_key_splits(int64_t Lq, int64_t Lk, int heads);
  * Stands in for the reference's dequantize-every-block-then-attend sequence: dequantize_kv_cache on all
  * max_blocks blocks of K and of V (utils/quant.py:731-768, utils/kernel/kv_dequant_cuda.cu:59-107; call
  * sites wan_5b/modules/causal_model.py:557-600, 628-652), window assembly with torch.cat (:673-724) and
- * attention() (:781, wan_5b/modules/attention.py:241-254).  Here the cached keys and values are decoded
- * inside the attention kernel's load stage, with the rounding of the fused dequantize kernel
- * (LLNV_DEQ_FUSED), so no bf16 copy of the cache exists and the result equals llnv_kv_dequant followed
- * by llnv_attention_bf16_ex on the concatenated window bit for bit.
+ * attention() (:781, wan_5b/modules/attention.py:241-254).  Here one launch expands the cached keys and
+ * values of all blocks into the workspace, with the rounding of the fused dequantize kernel (LLNV_DEQ_FUSED),
+ * and the attention kernel reads them there and the current chunk in place; the result equals llnv_kv_dequant
+ * followed by llnv_attention_bf16_ex on the concatenated window bit for bit.
  *   k_codes / k_sf / k_amax / v_*: HOST arrays of num_blocks (<= 16) DEVICE pointers, passed to the kernel
- *   as launch parameters.  Codes must be 16-byte aligned, block_token_size >= 128 (a 128-key tile then
- *   touches at most two blocks) and heads * 64 a multiple of 16.  num_blocks == 0 is llnv_attention_bf16_ex on
- *   the current chunk.  key_splits / workspace / out_amax as in llnv_attention_bf16_ex, with
- *   Lk = num_blocks * block_token_size + L_cur. */
+ *   as launch parameters.  Codes must be 16-byte aligned, block_token_size >= 128.  num_blocks == 0 is llnv_attention_bf16_ex on
+ *   the current chunk.  key_splits / out_amax as in llnv_attention_bf16_ex, with
+ *   Lk = num_blocks * block_token_size + L_cur; workspace: llnv_attention_nvfp4kv_workspace_bytes. */
 int llnv_attention_nvfp4kv(const void* q, int64_t Lq, int64_t ldq, const void* const* k_codes, const void* const* k_sf,
                            const float* const* k_amax, const void* const* v_codes, const void* const* v_sf,
                            const float* const* v_amax, int num_blocks, int block_token_size, float e2m1_max,
@@ -317,6 +316,9 @@ int llnv_attention_nvfp4kv(const void* q, int64_t Lq, int64_t ldq, const void* c
                            int heads, float scale, void* out, int64_t ldo, int key_splits, void* workspace,
                            int64_t workspace_bytes, float* out_amax, llnv_stream_t stream);
 int64_t llnv_attention_workspace_bytes(int64_t Lq, int heads, int key_splits);
+/* Workspace of an llnv_attention_nvfp4kv call: the partial results of a split call plus the cached blocks expanded to bf16.
+ * With less (down to llnv_attention_workspace_bytes) the call takes the expanded window from the stream-ordered allocator. */
+int64_t llnv_attention_nvfp4kv_workspace_bytes(int64_t Lq, int heads, int key_splits, int num_blocks, int block_token_size);
 
 /* Fused epilogue of the W4A4 GEMM.  All pointers are device pointers and optional (NULL = skip).
  * With everything NULL/0 the GEMM writes bf16(alpha * acc), which is what the reference's

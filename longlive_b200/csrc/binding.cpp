@@ -271,11 +271,11 @@ Tensor linear_nvfp4(const Tensor& input, int a_rule, const Tensor& w_codes, cons
 }
 
 // ---- attention ------------------------------------------------------------------------------------
-// The workspace of a split or tail-balanced call: the caller's, or a fresh one.
-OptTensor attention_workspace(int64_t lq, int heads, int key_splits, const OptTensor& workspace, const Tensor& q) {
-  if (!(key_splits > 1 || key_splits == LLNV_ATTN_SPLIT_TAIL)) return std::nullopt;
+// The workspace of a call: the caller's (which has to hold at least the partial results of a split), or a fresh one of
+// `want` bytes.
+OptTensor attention_workspace(int64_t lq, int heads, int key_splits, int64_t want, const OptTensor& workspace, const Tensor& q) {
   const int64_t bytes = llnv_attention_workspace_bytes(lq, heads, key_splits);
-  if (!workspace) return empty(q, {bytes}, at::kByte);
+  if (!workspace) return want > 0 ? OptTensor(empty(q, {want}, at::kByte)) : std::nullopt;
   if (workspace->scalar_type() != at::kByte || !workspace->is_contiguous() || workspace->numel() < bytes || workspace->device() != q.device())
     fail("attention workspace must be a contiguous uint8 tensor of at least " + std::to_string(bytes) + " bytes on the device of q");
   return workspace;
@@ -296,7 +296,7 @@ Tensor attention_bf16(const Tensor& q, const Tensor& k, const Tensor& v, int hea
   const int64_t lq = q.size(0), lk = k.size(0);
   if (!out) out = empty(q, {lq, (int64_t)heads * 128}, at::kBFloat16);
   const int splits = key_splits ? *key_splits : llnv_attention_key_splits(lq, lk, heads);
-  const OptTensor ws = attention_workspace(lq, heads, splits, workspace, q);
+  const OptTensor ws = attention_workspace(lq, heads, splits, llnv_attention_workspace_bytes(lq, heads, splits), workspace, q);
   check(llnv_attention_bf16_ex(ptr(q), lq, q.stride(0), ptr(k), ptr(v), lk, k.stride(0), v.stride(0), heads, (float)scale.value_or(kDefaultScale),
                                ptr(out), out->stride(0), splits, ptr(ws), ws ? ws->numel() : 0, fptr(out_amax), call.stream));
   return *out;
@@ -353,7 +353,8 @@ Tensor attention_nvfp4kv(const Tensor& q, const py::sequence& k_blocks, const py
   const int64_t lq = q.size(0), lk = (int64_t)n * block_tokens + l_cur;
   if (!out) out = empty(q, {lq, (int64_t)heads * 128}, at::kBFloat16);
   const int splits = key_splits ? *key_splits : llnv_attention_key_splits(lq, lk, heads);
-  const OptTensor ws = attention_workspace(lq, heads, splits, workspace, q);
+  const OptTensor ws =
+      attention_workspace(lq, heads, splits, llnv_attention_nvfp4kv_workspace_bytes(lq, heads, splits, n, block_tokens), workspace, q);
   check(llnv_attention_nvfp4kv(ptr(q), lq, q.stride(0), n ? kb.codes.data() : nullptr, n ? kb.sf.data() : nullptr, n ? kb.amax.data() : nullptr,
                                n ? vb.codes.data() : nullptr, n ? vb.sf.data() : nullptr, n ? vb.amax.data() : nullptr, n, block_tokens,
                                (float)e2m1_max, (float)e4m3_max, l_cur ? ptr(k_cur) : nullptr, l_cur ? ptr(v_cur) : nullptr, l_cur,

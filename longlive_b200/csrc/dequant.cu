@@ -1,6 +1,5 @@
 // NVFP4 -> bf16/fp16/fp32 dequantize: a general matrix form and the multi-block KV-cache form
 // (one launch for all cache blocks of a layer, pointer table passed as launch parameters).
-// Each thread decodes one 16-element block: one 8-byte code load, one scale byte, 32 bytes out.
 #include <cuda_fp4.h>
 
 #include "common.cuh"
@@ -10,10 +9,20 @@ namespace {
 
 constexpr int kMaxBlocks = 32;
 
+// Cache blocks of one launch: each with its own destination (a contiguous [rows, 128] matrix).
 struct BlockTable {
   const uint8_t* codes[kMaxBlocks];
   const uint8_t* sf[kMaxBlocks];
   const float* amax[kMaxBlocks];
+  void* out[kMaxBlocks];
+};
+
+// Rows of a bf16 matrix copied behind the blocks by the same launch (kv_window_dequant): up to two matrices.
+struct RowCopies {
+  const uint16_t* src[2];
+  uint16_t* dst[2];
+  int64_t ld[2];
+  int rows, cols;
 };
 
 template <int ROUNDING>
@@ -48,6 +57,25 @@ __device__ __forceinline__ void store16<float>(float* out, const float (&v)[16])
 #pragma unroll
   for (int i = 0; i < 4; ++i)
     reinterpret_cast<float4*>(out)[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+}
+
+template <typename T>
+__device__ __forceinline__ void store8(T* out, const float (&v)[8]);
+template <>
+__device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16* out, const float (&v)[8]) {
+  *reinterpret_cast<uint4*>(out) = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+}
+template <>
+__device__ __forceinline__ void store8<__half>(__half* out, const float (&v)[8]) {
+  __half2 h[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) h[i] = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+  *reinterpret_cast<uint4*>(out) = *reinterpret_cast<uint4*>(&h[0]);
+}
+template <>
+__device__ __forceinline__ void store8<float>(float* out, const float (&v)[8]) {
+  reinterpret_cast<float4*>(out)[0] = make_float4(v[0], v[1], v[2], v[3]);
+  reinterpret_cast<float4*>(out)[1] = make_float4(v[4], v[5], v[6], v[7]);
 }
 
 // decode 8 packed bytes (16 codes) and scale them
@@ -94,24 +122,60 @@ __global__ void __launch_bounds__(256) dequant_matrix_kernel(const uint8_t* __re
   }
 }
 
-// KV cache: block b holds `rows` logical rows of 128 columns; out row = b*rows + r.
+// KV cache: block b holds `rows` logical rows of 128 columns.
+//
+// Bound by HBM writes (2 bytes out for 9/16 in).  A lane decodes one code word = 8 values = one 16-byte store, so a warp's
+// store covers 512 contiguous bytes (with 16 values a thread the two halves of a sector came from two instructions and cost
+// two partial writes); a CTA of 256 threads covers 16 rows a step and takes kKvSteps steps whose loads are issued together.
+// 4 blocks of 2640 x 24 rows (8 with keys and values): see the entry points.
+constexpr int kKvSteps = 4;
+constexpr int kKvRows = 16 * kKvSteps;
 template <typename T, int ROUNDING>
-__global__ void __launch_bounds__(256) dequant_kv_kernel(BlockTable tab, int num_blocks, int64_t rows, float denom,
-                                                         T* __restrict__ out) {
+__global__ void __launch_bounds__(256) dequant_kv_kernel(const __grid_constant__ BlockTable tab, int num_blocks, int64_t rows, float denom,
+                                                         const __grid_constant__ RowCopies copies) {
   pdl_wait();
-  const int64_t per_block = rows * 8;
-  const int64_t total = per_block * num_blocks;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int b = (int)(i / per_block);
-    const int64_t j = i - (int64_t)b * per_block;
-    const int64_t r = j >> 3, c = j & 7;
-    const float amax = __ldg(tab.amax[b]);
-    const float g = global_scale(ROUNDING, amax, denom);
-    const uint2 p = __ldg(reinterpret_cast<const uint2*>(tab.codes[b] + r * 64 + c * 8));
-    const float s = e4m3_to_float(__ldg(tab.sf[b] + sf_offset(r, c, 8)));
-    float v[16];
-    decode16<ROUNDING>(p, s, amax, g, denom, v);
-    store16<T>(out + ((int64_t)b * rows + r) * 128 + c * 16, v);
+  const int b = blockIdx.y;
+  if (b >= num_blocks) {                                    // rows copied behind the blocks
+    const int m = b - num_blocks;
+    const int vecs = copies.cols / 8;
+    const int64_t total = (int64_t)copies.rows * vecs;
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
+      const int64_t r = i / vecs;
+      const int c = (int)(i - r * vecs);
+      reinterpret_cast<uint4*>(copies.dst[m])[i] = __ldg(reinterpret_cast<const uint4*>(copies.src[m] + r * copies.ld[m]) + c);
+    }
+    return;
+  }
+  const int c = threadIdx.x & 15;                            // code word of the row: columns 8c .. 8c + 7
+  const int64_t r0 = (int64_t)blockIdx.x * kKvRows + (threadIdx.x >> 4);
+  const uint32_t* codes = reinterpret_cast<const uint32_t*>(tab.codes[b]);
+  const uint8_t* sf = tab.sf[b];
+  uint32_t w[kKvSteps], sb[kKvSteps];
+#pragma unroll
+  for (int k = 0; k < kKvSteps; ++k) {
+    const int64_t r = r0 + 16 * k;
+    w[k] = sb[k] = 0u;
+    if (r < rows) {
+      w[k] = __ldg(codes + r * 16 + c);
+      sb[k] = __ldg(sf + sf_offset(r, c >> 1, 8));
+    }
+  }
+  const float amax = __ldg(tab.amax[b]);
+  const float g = global_scale(ROUNDING, amax, denom);
+  T* out = (T*)tab.out[b];
+#pragma unroll
+  for (int k = 0; k < kKvSteps; ++k) {
+    const int64_t r = r0 + 16 * k;
+    if (r >= rows) continue;
+    const float s = e4m3_to_float(sb[k]);
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __half2_raw h2 = __nv_cvt_fp4x2_to_halfraw2((__nv_fp4x2_storage_t)(uint8_t)(w[k] >> (8 * i)), __NV_E2M1);
+      v[2 * i] = deq_scale<ROUNDING>(__fmul_rn(__half2float(__ushort_as_half(h2.x)), s), amax, g, denom);
+      v[2 * i + 1] = deq_scale<ROUNDING>(__fmul_rn(__half2float(__ushort_as_half(h2.y)), s), amax, g, denom);
+    }
+    store8<T>(out + r * 128 + c * 8, v);
   }
 }
 
@@ -133,21 +197,45 @@ int launch_matrix(const uint8_t* codes, const uint8_t* sf, const float* amax, in
 }
 
 template <typename T>
-int launch_kv(const BlockTable& tab, int n, int64_t rows, float denom, int rounding, T* out, cudaStream_t stream) {
-  const int64_t total = rows * 8 * n;
-  if (total == 0) return LLNV_OK;
-  int64_t blocks = (total + 255) / 256;
-  const int64_t cap = (int64_t)sm_count() * 16;
-  if (blocks > cap) blocks = cap;
+int launch_kv(const BlockTable& tab, int n, int64_t rows, float denom, int rounding, const RowCopies& copies, cudaStream_t stream) {
+  const int extra = copies.rows > 0 ? 2 : 0;
+  if (rows * n == 0 && extra == 0) return LLNV_OK;
+  const int64_t gx = (rows + kKvRows - 1) / kKvRows;
+  LLNV_REQUIRE(gx < ((int64_t)1 << 31), "llnv_kv_dequant: too many rows (%lld)", (long long)rows);
+  const dim3 grid((unsigned)gx, (unsigned)(n + extra));
   switch (rounding) {
-    case LLNV_DEQ_FUSED: launch_k(dequant_kv_kernel<T, LLNV_DEQ_FUSED>, (unsigned)blocks, 256, 0, stream, tab, n, rows, denom, out); break;
-    case LLNV_DEQ_PYTORCH: launch_k(dequant_kv_kernel<T, LLNV_DEQ_PYTORCH>, (unsigned)blocks, 256, 0, stream, tab, n, rows, denom, out); break;
-    default: launch_k(dequant_kv_kernel<T, LLNV_DEQ_TRITON>, (unsigned)blocks, 256, 0, stream, tab, n, rows, denom, out); break;
+    case LLNV_DEQ_FUSED: launch_k(dequant_kv_kernel<T, LLNV_DEQ_FUSED>, grid, 256, 0, stream, tab, n, rows, denom, copies); break;
+    case LLNV_DEQ_PYTORCH: launch_k(dequant_kv_kernel<T, LLNV_DEQ_PYTORCH>, grid, 256, 0, stream, tab, n, rows, denom, copies); break;
+    default: launch_k(dequant_kv_kernel<T, LLNV_DEQ_TRITON>, grid, 256, 0, stream, tab, n, rows, denom, copies); break;
   }
   return launch_status("dequant_kv_kernel");
 }
 
 }  // namespace
+
+// Keys and values of the cached part of an attention window as bf16 [tokens, heads * 128] matrices (FUSED rounding), with
+// n_pad rows of the current chunk copied behind them so that the attention kernel's last tile of the cached part is whole.
+int kv_window_dequant(const void* const* k_codes, const void* const* k_sf, const float* const* k_amax, const void* const* v_codes,
+                      const void* const* v_sf, const float* const* v_amax, int num_blocks, int heads, int block_tokens, float denom,
+                      const void* k_cur, const void* v_cur, int64_t ldk, int64_t ldv, int n_pad, void* k_out, void* v_out, cudaStream_t stream) {
+  const int64_t rows = (int64_t)heads * block_tokens;
+  BlockTable tab;
+  for (int b = 0; b < num_blocks; ++b)
+    for (int m = 0; m < 2; ++m) {
+      const int i = 2 * b + m;
+      tab.codes[i] = (const uint8_t*)(m ? v_codes : k_codes)[b];
+      tab.sf[i] = (const uint8_t*)(m ? v_sf : k_sf)[b];
+      tab.amax[i] = (m ? v_amax : k_amax)[b];
+      tab.out[i] = (uint16_t*)(m ? v_out : k_out) + (int64_t)b * rows * 128;
+    }
+  RowCopies copies = {};
+  if (n_pad > 0)
+    copies = RowCopies{{(const uint16_t*)k_cur, (const uint16_t*)v_cur},
+                       {(uint16_t*)k_out + (int64_t)num_blocks * rows * 128, (uint16_t*)v_out + (int64_t)num_blocks * rows * 128},
+                       {ldk, ldv}, n_pad, heads * 128};
+  return launch_kv<__nv_bfloat16>(tab, 2 * num_blocks, rows, denom, LLNV_DEQ_FUSED, copies, stream);
+}
+
 }  // namespace llnv
 
 using namespace llnv;
@@ -199,12 +287,12 @@ extern "C" int llnv_kv_dequant(const void* const* codes, const void* const* sf, 
       tab.codes[i] = (const uint8_t*)codes[base + i];
       tab.sf[i] = (const uint8_t*)sf[base + i];
       tab.amax[i] = amax[base + i];
+      tab.out[i] = (char*)out + (size_t)(base + i) * rows * 128 * esize;
     }
-    char* o = (char*)out + (size_t)base * rows * 128 * esize;
     int rc;
-    if (dtype_code == LLNV_DTYPE_BF16) rc = launch_kv<__nv_bfloat16>(tab, n, rows, denom, rounding, (__nv_bfloat16*)o, stream);
-    else if (dtype_code == LLNV_DTYPE_FP16) rc = launch_kv<__half>(tab, n, rows, denom, rounding, (__half*)o, stream);
-    else rc = launch_kv<float>(tab, n, rows, denom, rounding, (float*)o, stream);
+    if (dtype_code == LLNV_DTYPE_BF16) rc = launch_kv<__nv_bfloat16>(tab, n, rows, denom, rounding, RowCopies{}, stream);
+    else if (dtype_code == LLNV_DTYPE_FP16) rc = launch_kv<__half>(tab, n, rows, denom, rounding, RowCopies{}, stream);
+    else rc = launch_kv<float>(tab, n, rows, denom, rounding, RowCopies{}, stream);
     if (rc != LLNV_OK) return rc;
   }
   return LLNV_OK;

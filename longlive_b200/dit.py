@@ -10,7 +10,7 @@ embedding, time/text MLPs and the head are plain bf16 torch ops (outside the hot
 Per block and forward (S tokens of the chunk, window = cached blocks + current chunk):
   adaLN(e0,e1)+quantize -> q,k,v GEMMs(+bias; v also emits its amax)
   -> RMSNorm+RoPE (q) / RMSNorm+RoPE+k_smooth+amax (k)
-  -> attention over [NVFP4 cache blocks, decoded inside the kernel | current chunk] -> quantize -> o GEMM(+bias,
+  -> attention over [NVFP4 cache blocks, expanded to bf16 by one launch | current chunk] -> quantize -> o GEMM(+bias,
   gate e2, residual) -> LayerNorm+quantize -> cross q GEMM -> RMSNorm -> attention over the text
   K/V -> quantize -> o GEMM(+bias, residual) -> adaLN(e3,e4)+quantize -> FFN GEMM(+bias, GELU, amax)
   -> quantize (amax given) -> FFN GEMM(+bias, gate e5, residual); then the rotated keys and the
@@ -243,8 +243,7 @@ class CausalDiT:
         self.cache_text_kv = cache_text_kv
         assert cfg.chunk_tokens % self.P == 0 and cfg.heads % self.P == 0, "tokens and heads must divide by the SP size"
         if cfg.chunk_tokens < 128:
-            raise ValueError("a cache block (one chunk) must hold at least 128 tokens: the attention kernel decodes 128-key tiles "
-                             "that may touch at most two blocks")
+            raise ValueError("a cache block (one chunk) must hold at least 128 tokens")
         gen = torch.Generator(device=self.device).manual_seed(seed)          # same weights on every rank
         self.blocks = [Block(cfg, gen, self.device) for _ in range(cfg.layers)]
         c = cfg.dim
@@ -275,10 +274,11 @@ class CausalDiT:
         self.q_buf, self.k_buf, self.v_buf = bf(Sl, c), bf(Sl, c), bf(Sl, c)
         self.q_rot, self.k_rot, self.k_smooth = bf(Sl, c), bf(Sl, c), bf(Sl, c)
         self.attn_out = bf(S, self.Cl)
-        # partial results of a split or tail-balanced self-attention call (none when the call is not split)
-        # (sized for every window length the cache passes through while it fills)
+        # self-attention: partial results of a split or tail-balanced call and the cached window in bf16, one buffer for all
+        # layers (sized for every window length the cache passes through while it fills)
         with torch.cuda.device(dev):
-            ws_bytes = max(ops.attention_workspace_bytes(S, n * cfg.chunk_tokens, self.Hl) for n in range(1, cfg.max_blocks + 1))
+            ws_bytes = max(ops.attention_nvfp4kv_workspace_bytes(S, n, cfg.chunk_tokens, cfg.chunk_tokens, self.Hl)
+                           for n in range(cfg.max_blocks))
         self.attn_ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev) if ws_bytes else None
         self.arena = None
         self.check_peer_status = True         # run_chunk raises ops.DeviceTimeout when a peer barrier gave up
@@ -306,10 +306,9 @@ class CausalDiT:
         self.cq_buf, self.cq_n = bf(Sl, c), bf(Sl, c)
         self.ck_buf, self.cv_buf, self.ck_n = bf(cfg.text_len, c), bf(cfg.text_len, c), bf(cfg.text_len, c)
         self.cattn = bf(Sl, c)
-        # The attention window is never materialised: the attention kernel decodes the NVFP4 cache blocks
-        # of the layer in its load stage and reads the current chunk's smoothed keys / values from cur_k /
-        # cur_v ([all chunk tokens, my heads], one pair shared by all layers; the reference dequantizes every
-        # block into a bf16 window per layer and forward, causal_model.py:557-600).
+        # The attention window: the cached blocks of the layer are expanded to bf16 into attn_ws, which all layers share, and the
+        # current chunk's smoothed keys / values are read from cur_k / cur_v ([all chunk tokens, my heads], one pair for all
+        # layers; the reference dequantizes every block into a bf16 window per layer and forward, causal_model.py:557-600).
         self.h_amax = torch.zeros(1, dtype=torch.float32, device=dev)
         # single-pass FFN requantization: per layer the amax the epilogue scales the hidden with (that of the layer's
         # previous forward) and the amax this forward measures

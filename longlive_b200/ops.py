@@ -261,6 +261,15 @@ def attention_workspace_bytes(lq, lk, heads, key_splits=None):
     return int(lib.llnv_attention_workspace_bytes(lq, heads, key_splits)) if (key_splits > 1 or key_splits == SPLIT_TAIL) else 0
 
 
+def attention_nvfp4kv_workspace_bytes(lq, blocks, block_tokens, l_cur, heads, key_splits=None):
+    """Bytes of workspace ``attention_nvfp4kv`` uses for ``blocks`` cached blocks and a current chunk of ``l_cur`` tokens
+    (``llnv_attention_nvfp4kv_workspace_bytes``)."""
+    lib = _lib.lib()
+    if key_splits is None:
+        key_splits = lib.llnv_attention_key_splits(lq, blocks * block_tokens + l_cur, heads)
+    return int(lib.llnv_attention_nvfp4kv_workspace_bytes(lq, heads, key_splits, blocks, block_tokens))
+
+
 def attention_bf16(q, k, v, heads, scale=None, out=None, key_splits=None, out_amax=None, workspace=None):
     """softmax(q k^T * scale) v per head, non-causal.  q: bf16 [Lq, heads*128]; k, v: bf16 [Lk, heads*128]
     (row strides free, unit column stride).  Returns bf16 [Lq, heads*128].  ``key_splits`` > 1 splits
@@ -273,8 +282,8 @@ def attention_bf16(q, k, v, heads, scale=None, out=None, key_splits=None, out_am
 
 def attention_nvfp4kv(q, k_blocks, v_blocks, block_tokens, k_cur, v_cur, heads, scale=None, out=None, key_splits=None,
                       out_amax=None, e2m1_max=6.0, e4m3_max=256.0, workspace=None):
-    """Chunk attention over [cached NVFP4 blocks ... | current chunk (bf16)] without dequantizing the cache to
-    memory (``llnv_attention_nvfp4kv``).  ``k_blocks`` / ``v_blocks``: cache blocks oldest first, each with
+    """Chunk attention over [cached NVFP4 blocks ... | current chunk (bf16)] (``llnv_attention_nvfp4kv``): the cached part is
+    expanded to bf16 in the workspace and attended from there, the current chunk is read in place.  ``k_blocks`` / ``v_blocks``: cache blocks oldest first, each with
     ``values`` (uint8 [rows_padded, 64]), ``scale_factors`` and ``amax`` (a ``QuantizedTensor`` of
     ``block_tokens * heads`` rows of 128 channels, token-major / head-minor).  ``k_cur`` / ``v_cur``: bf16
     [L_cur, heads*128] (or None when the window is the cache alone).  Result: bf16 [Lq, heads*128], equal bit

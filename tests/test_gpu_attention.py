@@ -340,3 +340,27 @@ def test_attention_caller_owned_workspace():
     assert torch.equal(a, b)
     with pytest.raises(RuntimeError, match="workspace"):
         ops.attention_bf16(q, k, v, 2, key_splits=4, workspace=ws[: need - 16])
+
+
+@pytest.mark.parametrize("T,blocks,l_cur,splits", [
+    (128, 2, 128, 1),        # the cached part fills whole key tiles: nothing of the current chunk is copied behind it
+    (144, 3, 80, 2),         # 80 rows complete the last tile of the cached part, none are left for the second tensors
+    (144, 3, 20, 1),         # fewer rows than the last tile has room for
+    (129, 1, 300, 3),        # one cached row in a tile of its own
+    (160, 2, 0, 1),          # no current chunk
+])
+def test_nvfp4kv_window_expansion_with_and_without_workspace(T, blocks, l_cur, splits):
+    """The expanded window in the caller's workspace and in stream-ordered memory (workspace for the splits only) give the same
+    result as dequantizing into a window and attending to it."""
+    heads, lq = 2, 270
+    g = torch.Generator(device="cuda").manual_seed(T + l_cur)
+    kq, vq = _cache_blocks(blocks, T, heads, g), _cache_blocks(blocks, T, heads, g)
+    q = torch.randn(lq, heads * 128, generator=g, device="cuda").bfloat16()
+    cur = [torch.randn(l_cur, heads * 128, generator=g, device="cuda").bfloat16() if l_cur else None for _ in range(2)]
+    ref = _dequant_then_attention(q, kq, vq, T, *cur, heads, key_splits=splits)
+    full = ops.attention_nvfp4kv_workspace_bytes(lq, blocks, T, l_cur, heads, key_splits=splits)
+    split = ops.attention_workspace_bytes(lq, blocks * T + l_cur, heads, key_splits=splits)
+    assert full > split
+    for n in (full, max(split, 16)):
+        ws = torch.full((n,), 0xFF, dtype=torch.uint8, device="cuda")
+        assert torch.equal(ops.attention_nvfp4kv(q, kq, vq, T, *cur, heads, key_splits=splits, workspace=ws), ref)
