@@ -51,11 +51,31 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-__device__ __forceinline__ float gelu_tanh(float x) {
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  const float u = k0 * (x + k1 * x * x * x);
-  return __fdividef(x, 1.f + __expf(-2.f * u));
+// GELU, tanh form, of two values: 0.5 x (1 + tanh(u)) = x / (1 + exp(-2u)), u = sqrt(2/pi) (x + 0.044715 x^3).  The constants are
+// folded into the exponent of exp2, x (c0 + c1 x^2): three packed multiplications, one packed addition and two
+// special-function instructions a value.  At +-inf and NaN it gives what the quotient gives.
+__device__ __forceinline__ F2 gelu_tanh2(F2 x) {
+  constexpr float c0 = (float)(-2.0 * 0.7978845608028654 * 1.4426950408889634), c1 = (float)(-2.0 * 0.7978845608028654 * 1.4426950408889634 * 0.044715);
+  const F2 a = f2_mul(x, f2_fma(f2_mul(x, x), f2_splat(c1), f2_splat(c0)));
+  F2 e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(a.x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(a.y));
+  e = f2_add(e, f2_splat(1.f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(e.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(e.y));
+  return f2_mul(x, r);
 }
+
+__device__ __forceinline__ F2 unpack2(uint32_t w) { return F2{bf16_lo(w), bf16_hi(w)}; }
+
+// larger magnitude of two packed bf16 pairs, lane by lane; a NaN lane gives way to the other operand
+__device__ __forceinline__ uint32_t amax_bf16x2(uint32_t running, uint32_t w) {
+  uint32_t d;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(running), "r"(w & 0x7FFF7FFFu));
+  return d;
+}
+// the larger lane of a packed running maximum (non-negative) as fp32
+__device__ __forceinline__ float amax_of_pair(uint32_t m) { return fmaxf(bf16_lo(m), bf16_hi(m)); }
 
 // epilogue variants (compile-time, so that the plain path stays a handful of instructions per
 // element and the whole epilogue fits the instruction cache)
@@ -79,7 +99,7 @@ __device__ __forceinline__ void drain_chunk(const uint32_t (&r)[2][32], float al
 template <int EPI>
 __device__ __forceinline__ void epilogue_packed(const uint32_t (&pk)[32], const uint16_t* __restrict__ bias,
                                                 const uint16_t* __restrict__ grow, int64_t col, uint8_t* buf, int lane,
-                                                bool want_amax, bool row_ok, float& local_amax, const QuantOut* qo = nullptr,
+                                                bool want_amax, bool row_ok, uint32_t& local_amax, const QuantOut* qo = nullptr,
                                                 bool store_bf16 = true) {
   constexpr bool has_res = (EPI & kEpiRes) != 0;
   constexpr bool has_quant = (EPI & kEpiQuant) != 0;
@@ -89,69 +109,48 @@ __device__ __forceinline__ void epilogue_packed(const uint32_t (&pk)[32], const 
 #pragma unroll
   for (int v8 = 0; v8 < 8; ++v8) {    // 8 columns (16 bytes) at a time
     uint4* slot = reinterpret_cast<uint4*>(buf + lane * 128 + ((v8 ^ (lane & 7)) << 4));
-    if (EPI == 0) {
-      if (want_amax && row_ok) {
+    uint4 ov = make_uint4(pk[v8 * 4], pk[v8 * 4 + 1], pk[v8 * 4 + 2], pk[v8 * 4 + 3]);
+    if (EPI & (kEpiBias | kEpiGelu | kEpiRes)) {
+      F2 y[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) y[e] = unpack2(pk[v8 * 4 + e]);
+      if (EPI & kEpiBias) {
+        const uint4 bv = __ldg(reinterpret_cast<const uint4*>(bias + col + v8 * 8));
+        const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          local_amax = fmaxf(local_amax, fmaxf(fabsf(bf16_lo(pk[v8 * 4 + e])), fabsf(bf16_hi(pk[v8 * 4 + e]))));
+          y[e] = f2_add(y[e], unpack2(bw[e]));
+          if (EPI & (kEpiGelu | kEpiRes)) round_bf16x2(y[e].x, y[e].y);
         }
       }
-      *slot = make_uint4(pk[v8 * 4], pk[v8 * 4 + 1], pk[v8 * 4 + 2], pk[v8 * 4 + 3]);
-      continue;
-    }
-    float y[8];
+      if (EPI & kEpiGelu) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      y[2 * e] = bf16_lo(pk[v8 * 4 + e]);
-      y[2 * e + 1] = bf16_hi(pk[v8 * 4 + e]);
-    }
-    if (EPI & kEpiBias) {
-      const uint4 bv = __ldg(reinterpret_cast<const uint4*>(bias + col + v8 * 8));
-      const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
-#pragma unroll
-      for (int e = 0; e < 8; e += 2) {
-        y[e] = y[e] + bf16_lo(bw[e >> 1]);
-        y[e + 1] = y[e + 1] + bf16_hi(bw[e >> 1]);
-        round_bf16x2(y[e], y[e + 1]);
-      }
-    }
-    if (EPI & kEpiGelu) {
-#pragma unroll
-      for (int e = 0; e < 8; e += 2) {
-        y[e] = gelu_tanh(y[e]);
-        y[e + 1] = gelu_tanh(y[e + 1]);
-        round_bf16x2(y[e], y[e + 1]);
-      }
-    }
-    if (has_res) {
-      const uint4 rv = *slot;
-      const uint32_t rw[4] = {rv.x, rv.y, rv.z, rv.w};
-      if (grow) {
-        const uint4 gv = __ldg(reinterpret_cast<const uint4*>(grow + col + v8 * 8));
-        const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
-#pragma unroll
-        for (int e = 0; e < 8; e += 2) {
-          y[e] = y[e] * bf16_lo(gw[e >> 1]);
-          y[e + 1] = y[e + 1] * bf16_hi(gw[e >> 1]);
-          round_bf16x2(y[e], y[e + 1]);
+        for (int e = 0; e < 4; ++e) {
+          y[e] = gelu_tanh2(y[e]);
+          if (has_res) round_bf16x2(y[e].x, y[e].y);
         }
       }
+      if (has_res) {
+        const uint4 rv = *slot;
+        const uint32_t rw[4] = {rv.x, rv.y, rv.z, rv.w};
+        if (grow) {
+          const uint4 gv = __ldg(reinterpret_cast<const uint4*>(grow + col + v8 * 8));
+          const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
 #pragma unroll
-      for (int e = 0; e < 8; e += 2) {
-        y[e] = bf16_lo(rw[e >> 1]) + y[e];
-        y[e + 1] = bf16_hi(rw[e >> 1]) + y[e + 1];
-        round_bf16x2(y[e], y[e + 1]);
+          for (int e = 0; e < 4; ++e) {
+            y[e] = f2_mul(y[e], unpack2(gw[e]));
+            round_bf16x2(y[e].x, y[e].y);
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] = f2_add(unpack2(rw[e]), y[e]);
       }
+      ov = make_uint4(pack2(y[0].x, y[0].y), pack2(y[1].x, y[1].y), pack2(y[2].x, y[2].y), pack2(y[3].x, y[3].y));
     }
     if (want_amax && row_ok) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) local_amax = fmaxf(local_amax, fabsf(y[e]));
+      // of the values as they are stored
+      local_amax = amax_bf16x2(amax_bf16x2(amax_bf16x2(amax_bf16x2(local_amax, ov.x), ov.y), ov.z), ov.w);
     }
-    uint4 ov;
-    ov.x = pack2(y[0], y[1]);
-    ov.y = pack2(y[2], y[3]);
-    ov.z = pack2(y[4], y[5]);
-    ov.w = pack2(y[6], y[7]);
     if (!has_quant || store_bf16) *slot = ov;
     if (has_quant) {
       // two 8-column units make one 16-element quantization block: the block quantizer of the standalone kernel,
@@ -172,16 +171,6 @@ __device__ __forceinline__ void epilogue_packed(const uint32_t (&pk)[32], const 
     reinterpret_cast<uint4*>(qo->codes)[1] = make_uint4(qc_words[4], qc_words[5], qc_words[6], qc_words[7]);
     *qo->sf = qsf;
   }
-}
-
-// Both steps for one chunk (kernels whose accumulators rotate drain and finish chunk by chunk).
-template <int EPI>
-__device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[2][32], float alpha, const uint16_t* __restrict__ bias,
-                                               const uint16_t* __restrict__ grow, int64_t col, uint8_t* buf, int lane,
-                                               bool want_amax, bool row_ok, float& local_amax) {
-  uint32_t pk[32];
-  drain_chunk(r, alpha, pk);
-  epilogue_packed<EPI>(pk, bias, grow, col, buf, lane, want_amax, row_ok, local_amax);
 }
 
 }  // namespace gemm

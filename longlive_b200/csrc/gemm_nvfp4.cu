@@ -3,7 +3,7 @@
 //
 //   D[M, N] = epilogue(alpha * A[M, K] * B[N, K]^T)
 //
-// One persistent CTA per SM, 6 warps:
+// One persistent CTA per SM, 10 warps:
 //   warp 0      TMA producer: per 256-element K block it loads the A tile (128 rows x 128 bytes of
 //               packed codes), the B tile (BN rows x 128 bytes) with the 128-byte swizzle, and the
 //               scale factors of both tiles (already stored as 512-byte 128x4 atoms, so a tile's
@@ -12,8 +12,11 @@
 //               tcgen05.cp, then issues four K=64 MMAs per stage; tcgen05.commit releases the
 //               stage to the producer and, after the last K block, hands the accumulator to the
 //               epilogue.  Warp 1 also owns the TMEM allocation.
-//   warps 2-5   epilogue: tcgen05.ld of the fp32 accumulator (32 lanes x 32 columns per load),
-//               alpha / bias / GELU / gate*y + residual / amax, bf16 stores.
+//   warps 2-9   epilogue: tcgen05.ld of the fp32 accumulator (32 lanes x 32 columns per load),
+//               alpha / bias / GELU / gate*y + residual / amax, bf16 stores.  Two warps per 32 rows of the
+//               tile, each with half of its columns: with four warps, one per scheduler, the epilogue of a 256-wide tile
+//               took longer than the twelve K blocks of K = 3072 (2640 x 14336 x 3072 with bias, GELU and amax 91 -> 62.5 us,
+//               2640 x 3072 x 3072 with bias, gate and residual 30.8 -> 21.1 us, with bias alone 20.0 -> 17.9 us).
 // BN = 128 and BN = 192 keep two accumulators in tensor memory so the epilogue of a tile overlaps
 // the main loop of the next one; BN = 256 has one accumulator (2 x 256 columns + scales exceed the
 // 512 columns) but the least shared-memory traffic per flop.  A 192-row B tile starts 0 or 64 rows
@@ -33,7 +36,7 @@ using namespace gemm;
 
 constexpr int BM = 128;
 constexpr int BK_BYTES = 128;            // 256 E2M1 elements
-constexpr int kThreads = 192;
+constexpr int kThreads = 320;
 constexpr uint32_t kTmemCols = 512;
 
 template <int BN>
@@ -47,12 +50,13 @@ struct Cfg {
   static constexpr uint32_t kSfbBytes = kSfbAtoms * 2048;
   static constexpr uint32_t kSfbColsPerK = 4 * kSfbAtoms;  // TMEM columns of B scales per K=64 MMA
   static constexpr uint32_t kStageBytes = kABytes + kBBytes + kSfaBytes + kSfbBytes;
-  // epilogue staging: per epilogue warp two buffers of 32 rows x 64 bf16 columns (128-byte rows,
-  // 128-byte swizzle) that TMA stores drain; the same buffers receive the residual tile first
-  // (the single-accumulator tile has one buffer per 64-column chunk, so that the residual of a whole
-  // tile can be fetched while its main loop still runs)
-  static constexpr int kBufs = kAcc == 1 ? BN / 64 : 2;
-  static constexpr uint32_t kStagingBytes = 4 * kBufs * 4096;
+  // epilogue staging: per epilogue warp one or two buffers of 32 rows x 64 bf16 columns (128-byte rows, 128-byte swizzle) that
+  // TMA stores drain; the same buffers receive the residual tile first (256-wide tiles have a buffer for each chunk a warp
+  // finishes, so that its residual can be fetched while the main loop still runs)
+  static constexpr int kChunks = BN / 64;
+  static constexpr int kOwn = (kChunks + 1) / 2;         // most chunks of a tile one warp finishes
+  static constexpr int kBufs = BN == 256 ? 2 : 1;
+  static constexpr uint32_t kStagingBytes = 8 * kBufs * 4096;
   static constexpr uint32_t kStagingOff = kStages * kStageBytes;
   static constexpr uint32_t kBarOff = kStagingOff + kStagingBytes;
   static constexpr uint32_t kSmemBytes = kBarOff + 1024;
@@ -63,7 +67,6 @@ struct Cfg {
   static_assert(kSfbCol + 4 * kSfbColsPerK <= kTmemCols, "tensor memory overflow");
 };
 
-// GELU, tanh form: 0.5 x (1 + tanh(u)) = x / (1 + exp(-2u)), u = sqrt(2/pi) (x + 0.044715 x^3)
 template <int BN, int EPI>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -76,7 +79,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   uint64_t* empty_bar = full_bar + C::kStages;
   uint64_t* tfull_bar = empty_bar + C::kStages;
   uint64_t* tempty_bar = tfull_bar + C::kAcc;
-  uint64_t* res_bar = tempty_bar + C::kAcc;                 // [4 warps][2 buffers]
+  uint64_t* res_bar = tempty_bar + C::kAcc;                 // [8 warps][kBufs buffers]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(res_bar + 16);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
@@ -101,7 +104,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
     for (int i = 0; i < C::kAcc; ++i) {
       mbar_init(&tfull_bar[i], 1);
-      mbar_init(&tempty_bar[i], 4);
+      mbar_init(&tempty_bar[i], 8);
     }
     for (int i = 0; i < 16; ++i) mbar_init(&res_bar[i], 1);
     *abort_flag = 0u;
@@ -201,8 +204,9 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..5)
+    // ------------------------------------------------------------------ epilogue (warps 2..9)
     const int q = warp & 3;                           // TMEM lane quarter this warp may access
+    const int half = warp >= 6 ? 1 : 0;               // which of the quarter's two warps this is
     float alpha0, alpha1 = 0.f, alpha2 = 0.f;           // per weight group (one group unless p.group_cols)
     if (p.epi.alpha) alpha0 = __ldg(p.epi.alpha);
     else alpha0 = __fdiv_rn(__fmul_rn(__ldg(p.a_amax), __ldg(p.b_amax)), p.alpha_denom);
@@ -216,13 +220,13 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     const uint16_t* bias = reinterpret_cast<const uint16_t*>(p.epi.bias);
     constexpr bool has_res = (EPI & kEpiRes) != 0;
     const uint16_t* gate = reinterpret_cast<const uint16_t*>(p.epi.gate);
-    uint8_t* my_stage = smem + C::kStagingOff + q * C::kBufs * 4096;
-    uint64_t* my_res_bar = res_bar + q * C::kBufs;
+    uint8_t* my_stage = smem + C::kStagingOff + (warp - 2) * C::kBufs * 4096;
+    uint64_t* my_res_bar = res_bar + (warp - 2) * C::kBufs;
     uint32_t res_phase = 0u;                          // bit b = parity to wait for on buffer b
     int acc = 0;
     uint32_t acc_phase = 0;
-    uint32_t chunk = 0;                               // running chunk counter -> staging buffer
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+    uint32_t iter = 0;                                // tiles done
+    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++iter) {
       const int mt = tile % num_m, nt = tile / num_m;
       const int row0 = mt * BM + q * 32;              // first row of this warp
       const int64_t row = (int64_t)row0 + lane;
@@ -236,65 +240,70 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       const CUtensorMap* tm_out = grp == 0 ? &tmD : &gmaps.m[grp - 1];
       const float* amax_dst = grp == 0 ? p.group_amax[0] : (grp == 1 ? p.group_amax[1] : p.group_amax[2]);
       const bool want_amax = p.group_cols ? amax_dst != nullptr : p.epi.out_amax != nullptr;
-      float local_amax = 0.f;
-      if (C::kAcc == 1) {
-        // one buffer per chunk: once the previous tile's stores have read them, the residual of the
-        // whole tile is fetched while the main loop is still running
-        if (row0 < p.M && lane == 0) {
-          bulk_wait_read<0>();
-          if (has_res) {
+      uint32_t local_amax = 0u;                      // packed running maximum of |out|
+      // Chunks of this warp: the lower or upper two of four, one of two, and of three (192-wide tiles) the first and last or the
+      // middle one in turn.
+      const int chunk0 = BN == 256 ? 2 * half : (BN == 128 ? half : (half ^ (int)(iter & 1u)));
+      constexpr int kStep = BN == 192 ? 2 : 1;
+      const int n_own = BN == 192 ? 2 - chunk0 : C::kOwn;
+      auto fetch_residual = [&](int i) {                // of the i-th chunk, into its buffer
+        mbar_arrive_expect_tx(&my_res_bar[i % C::kBufs], 4096);
+        tma_load_2d(my_stage + (i % C::kBufs) * 4096, &tmR, nt * BN + (chunk0 + i * kStep) * 64, row0, &my_res_bar[i % C::kBufs]);
+      };
+      if (row0 < p.M && lane == 0) {
+        // once the previous tile's stores have read the buffers, residuals are fetched while the main loop is still running
+        bulk_wait_read<0>();
+        if (has_res) {
 #pragma unroll
-            for (int ci = 0; ci < C::kBufs; ++ci) {
-              mbar_arrive_expect_tx(&my_res_bar[ci], 4096);
-              tma_load_2d(my_stage + ci * 4096, &tmR, nt * BN + ci * 64, row0, &my_res_bar[ci]);
-            }
-          }
-        }
-        __syncwarp();
-      } else if (has_res && row0 < p.M) {
-        // residual tile of the first chunk can be fetched while the main loop is still running
-        const uint32_t b0 = chunk & 1u;
-        if (lane == 0) {
-          bulk_wait_read<1>();                        // the store that used this buffer two chunks ago has read it
-          mbar_arrive_expect_tx(&my_res_bar[b0], 4096);
-          tma_load_2d(my_stage + b0 * 4096, &tmR, nt * BN, row0, &my_res_bar[b0]);
+          for (int i = 0; i < C::kBufs; ++i) fetch_residual(i);
         }
       }
+      __syncwarp();
       mbar_wait(&tfull_bar[acc], acc_phase, abort_flag, p.status, 300u);
       tc_fence_after();
-      // everything after the accumulator has been drained: residual wait, epilogue math, staging, store
-      auto finish_chunk = [&](int c0, const uint32_t (&pkc)[32]) {
-        const uint32_t b = C::kAcc == 1 ? (uint32_t)(c0 >> 6) : (chunk & 1u);
+      // Drain all chunks of this warp first (alpha, round to bf16, pack: 32 registers per 64 columns) and hand the accumulator back
+      // to the MMA warp, so that main loops go on while the epilogue math, residual waits and stores are still in progress.
+      const uint32_t acc_tmem = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
+      uint32_t pk[C::kOwn][32];
+#pragma unroll
+      for (int i = 0; i < C::kOwn; ++i) {
+        if (i >= n_own) break;
+        uint32_t r[2][32];
+        tmem_ld32(acc_tmem + (chunk0 + i * kStep) * 64, r[0]);
+        tmem_ld32(acc_tmem + (chunk0 + i * kStep) * 64 + 32, r[1]);
+        tmem_ld_wait();
+        drain_chunk(r, alpha, pk[i]);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tempty_bar[acc]);
+#pragma unroll
+      for (int i = 0; i < C::kOwn; ++i) {
+        if (i >= n_own) break;
+        const int b = i % C::kBufs;
         uint8_t* buf = my_stage + b * 4096;
+        const int64_t col = (int64_t)nt * BN + (chunk0 + i * kStep) * 64;
         if (row0 < p.M) {
-          if (C::kAcc == 1) {
-            if (has_res) {
-              mbar_wait(&my_res_bar[b], (res_phase >> b) & 1u, abort_flag, p.status, 301u);
-              res_phase ^= 1u << b;
-            }
-          } else if (has_res) {
-            // prefetch the residual of the next chunk of this tile into the other buffer
-            if (c0 + 64 < BN && lane == 0) {
+          if (i >= C::kBufs) {                          // the buffer is used a second time in this tile
+            if (lane == 0) {
               bulk_wait_read<0>();
-              mbar_arrive_expect_tx(&my_res_bar[b ^ 1u], 4096);
-              tma_load_2d(my_stage + (b ^ 1u) * 4096, &tmR, nt * BN + c0 + 64, row0, &my_res_bar[b ^ 1u]);
+              if (has_res) fetch_residual(i);
             }
-            mbar_wait(&my_res_bar[b], (res_phase >> b) & 1u, abort_flag, p.status, 301u);
-            res_phase ^= 1u << b;
-          } else {
-            if (lane == 0) bulk_wait_read<1>();       // buffer b was last used two chunks ago
             __syncwarp();
           }
-          const int64_t col = (int64_t)nt * BN + c0;
+          if (has_res) {
+            mbar_wait(&my_res_bar[b], (res_phase >> b) & 1u, abort_flag, p.status, 301u);
+            res_phase ^= 1u << b;
+          }
           if constexpr ((EPI & kEpiQuant) != 0) {
             // codes [Mp, N/2] row-major; scales in 512-byte atoms of 128 rows x 4 scale columns (64 elements)
             QuantOut qo;
             qo.qc = qconsts;
             qo.codes = p.q_codes + row * (p.N >> 1) + (col >> 1);
             qo.sf = reinterpret_cast<uint32_t*>(p.q_sf + ((int64_t)mt * (p.N >> 6) + (col >> 6)) * 512 + (row & 31) * 16 + ((row & 127) >> 5) * 4);
-            epilogue_packed<EPI>(pkc, bias, grow, col, buf, lane, want_amax, row_ok, local_amax, &qo, p.store_bf16 != 0);
+            epilogue_packed<EPI>(pk[i], bias, grow, col, buf, lane, want_amax, row_ok, local_amax, &qo, p.store_bf16 != 0);
           } else {
-            epilogue_packed<EPI>(pkc, bias, grow, col, buf, lane, want_amax, row_ok, local_amax);
+            epilogue_packed<EPI>(pk[i], bias, grow, col, buf, lane, want_amax, row_ok, local_amax);
           }
           fence_proxy_async();
           __syncwarp();
@@ -304,61 +313,16 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           }
         } else if constexpr ((EPI & kEpiQuant) != 0) {
           // a group of 32 padding rows (M..Mp-1): zero codes and zero scales, as the standalone quantizer writes them
-          const int64_t col = (int64_t)nt * BN + c0;
           uint4* cz = reinterpret_cast<uint4*>(p.q_codes + row * (p.N >> 1) + (col >> 1));
           cz[0] = make_uint4(0u, 0u, 0u, 0u);
           cz[1] = make_uint4(0u, 0u, 0u, 0u);
           *reinterpret_cast<uint32_t*>(p.q_sf + ((int64_t)mt * (p.N >> 6) + (col >> 6)) * 512 + (row & 31) * 16 + ((row & 127) >> 5) * 4) = 0u;
         }
-      };
-      const uint32_t acc_tmem = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
-      if constexpr (C::kAcc == 1) {
-        // Single accumulator: drain all of it first (alpha, round to bf16, pack: 32 registers per 64
-        // columns) and hand it back to the MMA warp, so that the next tile's main loop runs while
-        // this tile's epilogue math, residual waits and stores are still in progress.
-        constexpr int kChunks = BN / 64;
-        uint32_t pk[kChunks][32];
-#pragma unroll
-        for (int ci = 0; ci < kChunks; ++ci) {
-          uint32_t r[2][32];
-          tmem_ld32(acc_tmem + ci * 64, r[0]);
-          tmem_ld32(acc_tmem + ci * 64 + 32, r[1]);
-          tmem_ld_wait();
-          drain_chunk(r, alpha, pk[ci]);
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&tempty_bar[acc]);
-#pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 64, ++chunk) {
-          finish_chunk(c0, pk[0]);
-          // rotate the packed chunks so that the rolled loop always reads pk[0] (static register indices)
-#pragma unroll
-          for (int ci = 0; ci + 1 < kChunks; ++ci)
-#pragma unroll
-            for (int i = 0; i < 32; ++i) pk[ci][i] = pk[ci + 1][i];
-        }
-      } else {
-#pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 64, ++chunk) {
-          uint32_t r[2][32];
-          tmem_ld32(acc_tmem + c0, r[0]);
-          tmem_ld32(acc_tmem + c0 + 32, r[1]);
-          tmem_ld_wait();
-          if (c0 + 64 == BN) {
-            // accumulator fully read: hand it back to the MMA warp before the math and the stores
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&tempty_bar[acc]);
-          }
-          uint32_t pkc[32];
-          drain_chunk(r, alpha, pkc);
-          finish_chunk(c0, pkc);
-        }
       }
-      if (grp == 0) amax0 = fmaxf(amax0, local_amax);
-      else if (grp == 1) amax1 = fmaxf(amax1, local_amax);
-      else amax2 = fmaxf(amax2, local_amax);
+      const float tile_amax = amax_of_pair(local_amax);
+      if (grp == 0) amax0 = fmaxf(amax0, tile_amax);
+      else if (grp == 1) amax1 = fmaxf(amax1, tile_amax);
+      else amax2 = fmaxf(amax2, tile_amax);
       if (++acc == C::kAcc) { acc = 0; acc_phase ^= 1u; }
     }
     if (lane == 0) bulk_wait<0>();
@@ -461,15 +425,25 @@ int gemm_run(const void* a_codes, const void* a_sf, const float* a_amax, int a_r
   if (M == 0) return LLNV_OK;
 
   const int64_t group_cols = groups > 1 ? N / groups : 0;
-  int bn = (N % 256 == 0 && (groups == 1 || group_cols % 256 == 0)) ? 256 : 128;
-  // few tokens (a sequence-parallel shard): 256-wide tiles would leave SMs idle, 128-wide tiles double the grid
-  if (bn == 256 && ((M + 127) / 128) * (N / 256) * 2 <= (int64_t)sm_count() + 8) bn = 128;
-  // less than one wave of 256-wide tiles: 192-wide ones fill more SMs (and overlap their epilogue
-  // with the next main loop); with more tiles the lower operand traffic of the 256-wide tile wins
-  else if (bn == 256 && N % 192 == 0 && (groups == 1 || group_cols % 192 == 0) && ((M + 127) / 128) * (N / 256) <= (int64_t)sm_count()) bn = 192;
+  // Tile width: the one with the least waves x (width + 64) - a wave lasts as long as a tile's operand stream, in which the 128 rows
+  // of A and their scales count as much as 64 columns beyond their MMA time.  us at
+  // K = 3072 with 128 / 192 / 256: 660 x 3072 8.6 / 10.4 / 10.4, 880 x 3072 14.1 / 13.7 / 14.4 (one wave of 112 192-wide tiles),
+  // 1320 x 3072 14.5 / 17.1 / 14.4 (192-wide needs a second wave), 2640 x 3072 21.7 / 24.7 / 21.1, 2640 x 14336 69.0 / - / 62.5.
+  auto fits = [&](int w) { return N % w == 0 && (groups == 1 || group_cols % w == 0); };
+  int bn = 128;
+  int64_t best = 0;
+  for (const int w : {256, 192, 128}) {
+    if (!fits(w)) continue;
+    const int64_t sms = sm_count() > 0 ? sm_count() : 1, waves = (((M + 127) / 128) * (N / w) + sms - 1) / sms;
+    const int64_t cost = waves * (w + 64);
+    if (best == 0 || cost < best) {
+      best = cost;
+      bn = w;
+    }
+  }
   if (tile == 128) bn = 128;
-  if (tile == 192 && N % 192 == 0 && (groups == 1 || group_cols % 192 == 0)) bn = 192;
-  if (tile == 256 && N % 256 == 0 && (groups == 1 || group_cols % 256 == 0)) bn = 256;
+  if (tile == 192 && fits(192)) bn = 192;
+  if (tile == 256 && fits(256)) bn = 256;
 
   const uint64_t mp = (uint64_t)((M + 127) / 128 * 128);
   CUtensorMap tmA, tmB;
@@ -519,7 +493,8 @@ int gemm_run(const void* a_codes, const void* a_sf, const float* a_amax, int a_r
     if (rc != LLNV_OK) return rc;
   }
   const int variant = (epi.bias ? kEpiBias : 0) | (epi.act == 1 ? kEpiGelu : 0) | (epi.residual ? kEpiRes : 0) | (requant ? kEpiQuant : 0);
-  // CTA pairs pay off when the K loop dominates (measured: +13..17 % at K = 14336, no gain at K = 3072)
+  // CTA pairs pay off when the K loop dominates: us with 256-wide tiles / pairs, bias + gate + residual: K = 14336 2640 x 3072
+  // 63.7 / 58.6, 660 x 3072 34.9 / 32.9 (128-wide tiles 22.7); K = 3072 2640 x 3072 21.1 / 22.8, 2640 x 14336 62.6 / 71.8
   const bool pair_ok = N % 256 == 0 && !requant;
   const bool pair_auto = tile == 0 && K >= 8192 && M >= 1024 && groups == 1;
   if (pair_ok && groups == 1 && (tile == 2 || pair_auto)) return gemm_nvfp4_pair(a_codes, a_sf, b_codes, b_sf, p, tmD, tmR, variant, stream);

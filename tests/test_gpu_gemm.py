@@ -342,3 +342,27 @@ def test_fp4_mma_rate_probe_runs_and_reports_its_flop():
     assert flop.value == 2.0 * 128 * 256 * 256 * 64 * sms
     with pytest.raises(Exception):
         _lib.check(lib.llnv_fp4_mma_rate(0, None, None))
+
+
+@pytest.mark.parametrize("tile", [128, 192, 256, 2])
+@pytest.mark.parametrize("m,n,k", [(1, 768, 256), (2600, 3072, 512)])
+def test_gemm_epilogue_chunks_over_many_tiles(m, n, k, tile):
+    """Every warp of the epilogue finishes its share of several tiles (2600 rows: up to four tiles a CTA, the last rows ragged): bias,
+    gate and residual are single bf16 operations, so the result equals the plain product followed by them bit for bit; a NaN
+    does not reach the reported maximum."""
+    xq, wq = L.quantize_to_fp4(util.config_activation(m, k, seed=m).cuda()), L.quantize_to_fp4(util.config_weight(n, k, seed=n).cuda())
+    g = torch.Generator().manual_seed(9)
+    bias, gate = torch.randn(n, generator=g).bfloat16().cuda(), torch.randn((m + 879) // 880, n, generator=g).bfloat16().cuda()
+    resid = torch.randn(m, n, generator=g).bfloat16().cuda()
+    resid[m // 2, 5] = float("nan")
+    args = (xq.values, xq.scale_factors, xq.amax, 3, wq.values, wq.scale_factors, wq.amax, 3, m, n, k)
+    base = ops.gemm_nvfp4(*args, tile=128)
+    check_close(base[:256], O.bf16_round(oracle_matmul(xq, wq, m, n, k)[:256]), k)
+    amax = torch.zeros(1, dtype=torch.float32, device="cuda")
+    y = ops.gemm_nvfp4(*args, bias=bias, residual=resid, gate=gate, frame_rows=880, out_amax=amax, tile=tile)
+    ref = resid + (base + bias) * gate.repeat_interleave(880, 0)[:m]
+    torch.cuda.synchronize()
+    assert _lib.lib().llnv_check_status(None) == 0, _lib.lib().llnv_last_error()
+    ok = ~ref.isnan()
+    assert int((~ok).sum()) == 1 and torch.equal(y[ok], ref[ok]) and bool(y[m // 2, 5].isnan())
+    assert float(amax.item()) == float(ref[ok].float().abs().max().item())
