@@ -151,6 +151,7 @@ __global__ void __launch_bounds__(256) quantize_nvfp4_kernel(const uint16_t* x, 
     codes = pr.codes2;
     sf = pr.sf2;
   }
+  constexpr bool kTransform = MODE != kPlain;
   float amax_val = *amax_ptr;
   unsigned int peer_epoch = 0u;
   if (pr.peer.world > 1) {
@@ -177,10 +178,14 @@ __global__ void __launch_bounds__(256) quantize_nvfp4_kernel(const uint16_t* x, 
   const bool col_ok = col < K;
   const int64_t xoff = pr.shard_cols ? (col / pr.shard_cols) * pr.shard_stride + col % pr.shard_cols : col;
 
+  // this thread's blocks are 32 rows apart: pointers are carried along instead of being formed from the row index
+  const uint16_t* xp = x + (row_base + r0) * ldx + xoff;
+  uint8_t* cp = codes + (row_base + r0) * (K >> 1) + (col >> 1);
+  const int64_t x_step = 32 * ldx, c_step = 16 * K;
+  const int rows_left = col_ok ? (int)min(M - row_base - r0, (int64_t)128) : 0;       // rows beyond M read as zeros
   auto load_block = [&](int i, uint32_t (&w)[8]) {
-    const int64_t r = row_base + r0 + 32 * i;
-    if (col_ok && r < M) {
-      const uint4* p = reinterpret_cast<const uint4*>(x + r * ldx + xoff);
+    if (32 * i < rows_left) {
+      const uint4* p = reinterpret_cast<const uint4*>(xp);
       const uint4 a = __ldg(p), b = __ldg(p + 1);
       w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
       w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
@@ -188,6 +193,7 @@ __global__ void __launch_bounds__(256) quantize_nvfp4_kernel(const uint16_t* x, 
 #pragma unroll
       for (int j = 0; j < 8; ++j) w[j] = 0u;
     }
+    xp += x_step;
   };
 
   uint32_t nxt[8];
@@ -199,8 +205,8 @@ __global__ void __launch_bounds__(256) quantize_nvfp4_kernel(const uint16_t* x, 
 #pragma unroll
     for (int j = 0; j < 8; ++j) cur[j] = nxt[j];
     if (i < 3) load_block(i + 1, nxt);
-    const int64_t r = row_base + r0 + 32 * i;
-    if (MODE != kPlain && col_ok && r < M) {
+    if (kTransform && 32 * i < rows_left) {
+      const int64_t r = row_base + r0 + 32 * i;
       transform_block<MODE>(cur, pr, r, col);
       if (y_out) {
         uint4* yo = reinterpret_cast<uint4*>(y_out + r * ldy + col);
@@ -208,14 +214,15 @@ __global__ void __launch_bounds__(256) quantize_nvfp4_kernel(const uint16_t* x, 
         yo[1] = make_uint4(cur[4], cur[5], cur[6], cur[7]);
       }
     }
-    if (codes == nullptr) continue;          // transform-only call (y_out): nothing to quantize
+    if (kTransform && codes == nullptr) continue;          // transform-only call (y_out): nothing to quantize
     uint32_t c_lo, c_hi, s;
     if (F16) quant_block_f16<RULE>(cur, qc, c_lo, c_hi, s);      // the words hold fp16 values
     else quant_block<RULE>(cur, qc, c_lo, c_hi, s);
-    if (col_ok) *reinterpret_cast<uint2*>(codes + r * (K >> 1) + (col >> 1)) = make_uint2(c_lo, c_hi);
+    if (col_ok) *reinterpret_cast<uint2*>(cp) = make_uint2(c_lo, c_hi);
+    cp += c_step;
     my_sf |= s << (8 * i);
   }
-  if (codes == nullptr) return;
+  if (kTransform && codes == nullptr) return;
 
   // Transpose the 4x4 scale bytes of each group of four lanes: lane q ends up with the word of
   // 16-byte unit r0 that holds row (r0 + 32*q), scale columns 4*(cb/4) .. +3.

@@ -232,3 +232,25 @@ def test_quantize_fp16_input(golden, rule):
         import longlive_b200.torch_ops  # noqa: F401  (registers torch.ops.llnvfp4)
         v, s, a = torch.ops.llnvfp4.quantize_to_fp4(big.cuda(), True, True, False, False, False, 3, 0)
         assert torch.equal(v, qb.values) and torch.equal(s.view(torch.uint8), qb.scale_factors.view(torch.uint8)) and torch.equal(a, qb.amax)
+
+
+@pytest.mark.parametrize("rule", RULES)
+@pytest.mark.parametrize("kind", ["lattice", "sparse", "row_scales", "negative_zero"])
+def test_quantize_close_decisions_match_oracle(rule, kind):
+    """Blocks whose two candidates have equal or nearly equal errors (values on a lattice, one or two values in a block, blocks far
+    below the tensor maximum) are decided as the reference's rounding decides them."""
+    g = torch.Generator().manual_seed(3)
+    x = torch.randn(384, 512, generator=g)
+    if kind == "lattice":
+        x = torch.round(x * 4) * 0.1875
+    elif kind == "sparse":
+        x = torch.where(torch.rand(x.shape, generator=g) < 0.9, torch.zeros(()), x)
+    elif kind == "row_scales":
+        x = x * torch.exp2(torch.randint(-14, 2, (384, 1), generator=g).float())
+    else:
+        x = torch.where(x.abs() < 0.5, -torch.zeros(()), x)
+    x = x.bfloat16()
+    q = L.quantize_to_fp4(x.cuda(), L.QuantizationConfig(scale_rule=rule))
+    codes, sf, amax = O.quantize_nvfp4(x.float().numpy(), rule)
+    assert float(q.amax.item()) == float(amax)
+    assert np.array_equal(util.u8(q.scale_factors), sf) and np.array_equal(q.values.cpu().numpy(), codes)
