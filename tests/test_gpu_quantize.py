@@ -254,3 +254,16 @@ def test_quantize_close_decisions_match_oracle(rule, kind):
     codes, sf, amax = O.quantize_nvfp4(x.float().numpy(), rule)
     assert float(q.amax.item()) == float(amax)
     assert np.array_equal(util.u8(q.scale_factors), sf) and np.array_equal(q.values.cpu().numpy(), codes)
+
+
+@pytest.mark.parametrize("m,k", [(1, 64), (42, 3072), (43, 3072), (2048, 64), (2049, 64), (700, 1088)])
+def test_quantize_amax_forms_agree(m, k):
+    """The amax taken inside the quantizer (up to 131072 elements), by the separate pass, and of rows that lie apart."""
+    x = util.config_activation(m, k, seed=m)
+    wide = torch.full((m, k + 8), 1e4, dtype=torch.bfloat16)
+    wide[:, :k] = x
+    codes, sf, amax = O.quantize_nvfp4(x.float().numpy(), "mse")
+    for t in (x.cuda(), wide.cuda()[:, :k]):
+        q = ops.quantize_nvfp4(t, 3)
+        assert float(q[2].item()) == float(amax) == float(ops.amax_bf16(t).item())
+        assert np.array_equal(util.u8(q[1]), sf) and np.array_equal(q[0].cpu().numpy(), codes)
