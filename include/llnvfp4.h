@@ -481,10 +481,10 @@ int llnv_unipc_step(const void* model_output, const void* sample, const void* x0
 /* Number of kernels the library has launched in this process (every launch, captured ones included, is counted
  * when it is issued; a replayed graph is not re-counted). */
 unsigned long long llnv_launch_count(void);
-/* 1: launch kernels with programmatic stream serialization (the next kernel of a stream is
- * scheduled while the previous one drains and waits for it on the device); 0 (default): plain
- * launches.  Returns the previous setting.  The environment variable LLNV_PDL=1 switches it on at
- * load time.  Results do not depend on it; on a B200 it measured no gain for graph-replayed chunks. */
+/* 1 (default): launch kernels with programmatic stream serialization (the next kernel of a stream is
+ * scheduled while the previous one drains and waits for it on the device); 0: plain
+ * launches.  Returns the previous setting.  The environment variable LLNV_PDL=0 switches it off at
+ * load time.  Results do not depend on it. */
 int llnv_set_pdl(int on);
 int llnv_selftest_div_const(int divisor, uint32_t first_bits, uint64_t count, unsigned long long* mismatches,
                             llnv_stream_t stream);

@@ -306,7 +306,6 @@ __global__ void __launch_bounds__(kThreads, 1)
 attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                  const __grid_constant__ CUtensorMap tmK2, const __grid_constant__ CUtensorMap tmV2, const __grid_constant__ CUtensorMap tmO,
                  const AttnParams p) {
-  pdl_wait();
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* q_full = reinterpret_cast<uint64_t*>(smem + kBarOff);
   uint64_t* k_full = q_full + 1;
@@ -324,10 +323,14 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const int qt = blockIdx.x, head = blockIdx.y;
   int j0, nt;
   bool partial;
-  if (!key_range(p, qt, head, j0, nt, partial)) return;          // nothing is set up yet: the CTA just leaves
+  if (!key_range(p, qt, head, j0, nt, partial)) {                // nothing is set up yet: the CTA just leaves
+    pdl_wait();
+    return;
+  }
   const int n_half = ((int64_t)qt * kBQ + kHQ < p.Lq) ? 2 : 1;     // the second half may lie entirely beyond Lq
 
   if ((smem_u32(smem) & 1023u) != 0) {
+    pdl_wait();
     if (threadIdx.x == 0 && p.status && atomicCAS(p.status, 0u, 2u) == 0u) p.status[1] = 901u;
     return;
   }
@@ -356,12 +359,14 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     prefetch_tensormap(&tmV2);
     prefetch_tensormap(&tmO);
   }
+  pdl_wait();
   if (warp == 1) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
+  pdl_trigger();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   // The register file is re-divided at the top of every warpgroup's branch (all four warps of a warpgroup execute the same
@@ -541,7 +546,7 @@ __global__ void __launch_bounds__(256) attention_combine_kernel(const float* __r
                                                                 int nsplit, int64_t Lq, int heads, float scale_log2,
                                                                 uint16_t* __restrict__ out, int64_t ldo, float* __restrict__ out_amax,
                                                                 int first_item, int q_tiles) {
-  pdl_wait();
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int item = first_item + (int)blockIdx.x / (kBQ / (8 * kCombineRows));
   const int head = item / q_tiles;

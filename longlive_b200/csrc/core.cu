@@ -59,7 +59,7 @@ void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 
 namespace {
 thread_local int g_amax_accumulate = 0;
-int g_pdl = -1;                        // -1: not decided yet (environment LLNV_PDL=1 turns it on; default off)
+int g_pdl = -1;                        // -1: not decided yet (on, unless the environment has LLNV_PDL=0)
 }
 
 bool amax_accumulate(int which) { return (g_amax_accumulate & which) != 0; }
@@ -67,7 +67,7 @@ bool amax_accumulate(int which) { return (g_amax_accumulate & which) != 0; }
 bool pdl_enabled() {
   if (g_pdl < 0) {
     const char* e = getenv("LLNV_PDL");
-    g_pdl = (e && e[0] == '1') ? 1 : 0;
+    g_pdl = (e && e[0] == '0') ? 0 : 1;
   }
   return g_pdl != 0;
 }

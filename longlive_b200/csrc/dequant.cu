@@ -107,7 +107,7 @@ template <typename T, int ROUNDING>
 __global__ void __launch_bounds__(256) dequant_matrix_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ sf,
                                                              const float* __restrict__ amax_ptr, int64_t rows, int64_t cols,
                                                              int64_t cols_padded, float denom, T* __restrict__ out, int64_t ldo) {
-  pdl_wait();
+  pdl_begin();
   const int64_t groups_per_row = cols >> 4;
   const int64_t total = rows * groups_per_row;
   const float amax = *amax_ptr;
@@ -133,7 +133,7 @@ constexpr int kKvRows = 16 * kKvSteps;
 template <typename T, int ROUNDING>
 __global__ void __launch_bounds__(256) dequant_kv_kernel(const __grid_constant__ BlockTable tab, int num_blocks, int64_t rows, float denom,
                                                          const __grid_constant__ RowCopies copies) {
-  pdl_wait();
+  pdl_begin();
   const int b = blockIdx.y;
   if (b >= num_blocks) {                                    // rows copied behind the blocks
     const int m = b - num_blocks;

@@ -72,7 +72,6 @@ __global__ void __launch_bounds__(kThreads, 1)
 gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                   const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmR,
                   const __grid_constant__ GroupMaps gmaps, const GemmParams p) {
-  pdl_wait();
   using C = Cfg<BN>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + C::kBarOff);
@@ -93,6 +92,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const int64_t k_atoms = p.K / 64;       // 512-byte scale atoms per 128-row tile
 
   if ((smem_u32(smem) & 1023u) != 0) {    // swizzled tiles need a 1024-byte aligned base
+    pdl_wait();
     if (threadIdx.x == 0 && p.status && atomicCAS(p.status, 0u, 2u) == 0u) p.status[1] = 900u;
     return;
   }
@@ -113,6 +113,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     prefetch_tensormap(&tmB);
     prefetch_tensormap(&tmD);
   }
+  pdl_wait();
   if (warp == 1) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
@@ -120,6 +121,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {

@@ -52,7 +52,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                        const __grid_constant__ CUtensorMap tmSFA, const __grid_constant__ CUtensorMap tmSFB,
                        const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmR, const GemmParams p) {
-  pdl_wait();
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kBarOff);     // used in the leader only
   uint64_t* empty_bar = full_bar + kStages;
@@ -76,6 +75,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
 
   if ((smem_u32(smem) & 1023u) != 0) {
     // both CTAs of a pair see the same alignment, so both leave here and nobody waits for the other
+    pdl_wait();
     if (threadIdx.x == 0 && p.status && atomicCAS(p.status, 0u, 2u) == 0u) p.status[1] = 902u;
     return;
   }
@@ -97,6 +97,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     prefetch_tensormap(&tmSFB);
     prefetch_tensormap(&tmD);
   }
+  pdl_wait();
   if (warp == 1) {
     tmem_alloc_pair(tmem_slot, kTmemCols);
     tmem_relinquish_pair();
@@ -105,6 +106,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   __syncthreads();
   cluster_sync();                                     // the peer's barriers are initialised from here on
   tc_fence_after();
+  pdl_trigger();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {

@@ -66,7 +66,6 @@ template <int BN>
 __global__ void __launch_bounds__(kThreadsLin, 1)
 linear_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const __grid_constant__ CUtensorMap tmD, const LinParams p) {
-  pdl_wait();
   using Cfg = LinCfg<BN>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -95,6 +94,7 @@ linear_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     prefetch_tensormap(&tmB);
     prefetch_tensormap(&tmD);
   }
+  pdl_wait();
   if (warp == 1) {
     tmem_alloc(tmem_slot, BN);
     tmem_relinquish();
@@ -102,6 +102,7 @@ linear_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {

@@ -82,7 +82,7 @@ __device__ __forceinline__ uint32_t cta_amax_bits(const uint16_t* __restrict__ x
 template <bool F16, bool ROWS>
 __global__ void __launch_bounds__(256) amax_16bit_kernel(const uint16_t* __restrict__ x, int64_t M, int64_t K,
                                                          int64_t ldx, float* __restrict__ amax) {
-  pdl_wait();
+  pdl_begin();
   const uint32_t mm = cta_amax_bits<ROWS>(x, M, K, ldx, blockIdx.x, gridDim.x);
   if (threadIdx.x == 0 && mm != 0) {
     const int bits = F16 ? __float_as_int(__half2float(__ushort_as_half((unsigned short)mm))) : (int)(mm << 16);
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(256) quantize_nvfp4_kernel(const uint16_t* x, 
                                                              int64_t ldx, const float* amax_ptr,
                                                              uint8_t* codes, uint8_t* sf,
                                                              const Prologue pr, uint16_t* __restrict__ y_out, int64_t ldy) {
-  pdl_wait();
+  pdl_begin();
   if (blockIdx.z == 1) {          // second tensor of a two-tensor launch
     x = pr.x2;
     amax_ptr = pr.amax2;
@@ -296,7 +296,7 @@ template <int MODE, int WPR>
 __global__ void __launch_bounds__(256, WPR > 1 ? 8 : 1) ln_stats_amax_kernel(const uint16_t* __restrict__ x, int64_t M, int64_t C, int64_t ldx,
                                                             float eps, Prologue pr, float* __restrict__ row_stats,
                                                             float* __restrict__ amax) {
-  pdl_wait();
+  pdl_begin();
   constexpr int kVec = 16 / WPR;              // 16-byte vectors per lane: C <= 4096
   constexpr int kRows = 8 / WPR;              // rows per CTA
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(256, WPR > 1 ? 8 : 1) ln_stats_amax_kernel(con
 // IEEE division (used by the test-suite to pin the range on which the fast path may rely on it).
 template <int D>
 __global__ void div_const_selftest_kernel(uint32_t first, uint64_t count, unsigned long long* mismatches) {
-  pdl_wait();
+  pdl_begin();
   unsigned long long bad = 0;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (uint64_t)gridDim.x * blockDim.x) {
     const float x = __uint_as_float(first + (uint32_t)i);

@@ -46,7 +46,7 @@ template <int WPR>
 __global__ void __launch_bounds__(256) rmsnorm_rope_kernel(const __grid_constant__ RopeJobs jobs, int64_t S, int64_t C, float eps,
                                                            const float* __restrict__ cosv, const float* __restrict__ sinv,
                                                            int shard_vecs) {
-  pdl_wait();
+  pdl_begin();
   const RopeJob& jb = jobs.job[blockIdx.y];
   const uint16_t* __restrict__ x = jb.x;
   const uint16_t* __restrict__ weight = jb.weight;

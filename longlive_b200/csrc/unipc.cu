@@ -110,7 +110,7 @@ struct Elem<false> {
 template <bool BF16, bool VEC>
 __global__ void __launch_bounds__(256) unipc_step_kernel(const void* v_, const void* x_, const void* m0_, const void* m1_, const void* last_,
                                                          void* x0_, void* xs_, void* next_, int64_t n, const __grid_constant__ Coef c) {
-  pdl_wait();
+  pdl_begin();
   using E = Elem<BF16>;
   using T = typename E::T;
   const T* v = (const T*)v_;
