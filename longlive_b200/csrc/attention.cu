@@ -173,9 +173,9 @@ __device__ __forceinline__ F2 ex2_poly2(F2 x) {
   pl = f2_fma(pl, f, f2_splat(1.f));
   return F2{__int_as_float(__float_as_int(pl.x) + (__float_as_int(r.x) << 23)), __int_as_float(__float_as_int(pl.y) + (__float_as_int(r.y) << 23))};
 }
-// Pair p of a row's scores takes the FMA-pipe exp2.  One pair in three: per 256 x 128 tile the special-function unit is then
-// busy 1360 cycles of about 2570, the FMA pipe 1010 and the issue slots 1300.  (2640 x 13200 x 24 heads, us: a quarter of the
-// pairs 350.5, a third 349.0, two fifths 356, half 368.)
+// Pair p of a row's scores takes the FMA-pipe exp2.  One pair in four: per 256 x 128 tile the special-function unit is then
+// busy 1540 cycles of about 2570.  (2640 x 13200 x 24 heads, us: a quarter of the pairs 350.5, a third 349.0, two fifths 356, half
+// 368: the quarter leaves the FMA pipe and the issue slots more room at the same time within the spread of runs.)
 __host__ __device__ constexpr bool poly_pair(int p) { return p % 4 == 1; }
 
 // Maximum of a row's scores: independent chains of three-input maxima.

@@ -42,6 +42,14 @@ __device__ __forceinline__ float2 e2m1x2_to_float2(uint32_t byte) {
   const __half2_raw h = __nv_cvt_fp4x2_to_halfraw2((__nv_fp4x2_storage_t)byte, __NV_E2M1);
   return __half22float2(*reinterpret_cast<const __half2*>(&h));
 }
+// two E2M1 codes minus two fp32 values (mixed-precision subtraction: the fp16 forms of the codes are exact and need no conversion)
+__device__ __forceinline__ F2 e2m1x2_minus(uint32_t byte, F2 t) {
+  const __half2_raw h = __nv_cvt_fp4x2_to_halfraw2((__nv_fp4x2_storage_t)byte, __NV_E2M1);
+  F2 d;
+  asm("sub.rn.f32.f16 %0, %1, %2;" : "=f"(d.x) : "h"(h.x), "f"(t.x));
+  asm("sub.rn.f32.f16 %0, %1, %2;" : "=f"(d.y) : "h"(h.y), "f"(t.y));
+  return d;
+}
 // two fp32 -> two E4M3 bytes (lo in bits 0-7), round to nearest even, saturating
 __device__ __forceinline__ uint32_t cvt_e4m3x2(float lo, float hi) {
   return (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(lo, hi), __NV_SATFINITE, __NV_E4M3);
@@ -234,7 +242,7 @@ __device__ __forceinline__ void quant_block(const uint32_t (&w)[8], const QuantC
   // block maximum on the packed 15-bit magnitudes
   uint32_t m = 0;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) m = __vmaxu2(m, w[j] & 0x7FFF7FFFu);
+  for (int j = 0; j < 8; j += 2) m = __vimax3_u16x2(m, w[j] & 0x7FFF7FFFu, w[j + 1] & 0x7FFF7FFFu);
   const float bmax = __uint_as_float(max(m & 0xFFFFu, m >> 16) << 16);
   float hp;
   if (qc.amax == 0.f) hp = 0.f;
@@ -280,8 +288,7 @@ __device__ __forceinline__ void quant_block(const uint32_t (&w)[8], const QuantC
     // candidate-6 and candidate-4 code bytes of this pair side by side; the selected ones are gathered at the end
     pa[j] = __byte_perm(k6, k4, 0x0040);
     if (!kEstimate) continue;
-    const float2 q6 = e2m1x2_to_float2(k6), q4 = e2m1x2_to_float2(k4);
-    const F2 d6 = f2_sub(F2{q6.x, q6.y}, t6), d4 = f2_sub(F2{q4.x, q4.y}, t4);
+    const F2 d6 = e2m1x2_minus(k6, t6), d4 = e2m1x2_minus(k4, t4);
     if (RULE == LLNV_RULE_MSE) {
       n6 = f2_fma(d6, d6, n6);
       n4 = f2_fma(d4, d4, n4);
