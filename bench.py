@@ -444,8 +444,8 @@ def attention_roofline(dev, rank, world, peaks, iters=8):
     achieved = fl / (ms * 1e-3) / 1e12
     peak = peaks["bf16_tflops"]
     return {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
-            "traffic": (lambda t: None if t is None else t * heads / 24.0)(dram_traffic("attention_kernel<fused>", "2640x4x2640x24")),
-            "traffic_case": "ncu capture at 24 heads (profiles/dram_traffic.md), scaled by heads / 24", "kernel": "attention_kernel behind one launch that expands the NVFP4 blocks to bf16",
+            "traffic": (lambda t: None if t is None else t * heads / 24.0)(dram_traffic("dequant_kv_kernel + attention_kernel", "2640x4x2640x24")),
+            "traffic_case": "ncu capture at 24 heads (profiles/dram_traffic.md), scaled by heads / 24; null: none of the present kernels", "kernel": "attention_kernel behind one launch that expands the NVFP4 blocks to bf16",
             "shape": f"{t} queries x {(blocks + 1) * t} keys x {heads} heads", "avg_launch_us": ms * 1e3, "launches_timed": iters,
             "algorithmic_flops_per_launch": fl,
             "peak_note": f"{peaks['source']} dense bf16 burst peak (cuBLAS GEMM); the kernel's MMAs are bf16 (kind::f16)"}
