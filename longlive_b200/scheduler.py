@@ -111,8 +111,11 @@ class FlowUniPCMultistepScheduler:
         """Sigma grid and integer timesteps of a run (fm_solvers_unipc.py:162-229); clears the step state."""
         if shift is None:
             shift = self.shift
-        # the grid of (steps, shift) is a host table of a few numbers; a video sets the same one for every chunk
-        key = (num_inference_steps, shift) if sigmas is None else None
+        # The grid is a host table of a few numbers; a video sets the same one for every chunk.  The key holds everything the grid is
+        # made of, and only plain numbers: their hash is their value (a tensor's is its identity), and 4 is not 4.0 to linspace.
+        key = (num_inference_steps, shift, self.sigma_max, self.sigma_min, self.num_train_timesteps)
+        if sigmas is not None or type(num_inference_steps) is not int or not all(type(v) in (int, float) for v in key):
+            key = None
         grid = self._grids.get(key) if key is not None else None
         if grid is None:
             if sigmas is None:

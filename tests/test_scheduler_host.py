@@ -102,3 +102,36 @@ def test_step_needs_set_timesteps_and_a_cuda_tensor():
     with pytest.raises(ValueError, match="CUDA tensor"):
         s.step(x, 999, x)                                               # CPU tensors: there is no CPU path
     assert s.index_for_timestep(833) == 2 and s.index_for_timestep(5) == 3
+
+
+def test_schedule_follows_everything_it_is_made_of():
+    """A second ``set_timesteps`` with the same arguments sees a changed ``sigma_max`` / ``sigma_min`` / ``num_train_timesteps``, and
+    what a caller writes into the returned tensors does not come back."""
+    s = _sched(4, 5.0)
+    assert s.timesteps.tolist() == [999, 937, 833, 624]
+    s.sigmas.zero_()
+    s.timesteps.zero_()
+    s.set_timesteps(4, shift=5.0)
+    assert s.timesteps.tolist() == [999, 937, 833, 624] and float(s.sigmas[0]) > 0.99
+    for name, value in (("sigma_max", 0.5), ("sigma_min", 0.25), ("num_train_timesteps", 500)):
+        setattr(s, name, value)
+        s.set_timesteps(4, shift=5.0)
+        x = np.linspace(s.sigma_max, s.sigma_min, 5)[:-1]
+        x = 5.0 * x / (1 + 4.0 * x)
+        assert s.timesteps.tolist() == (x * s.num_train_timesteps).astype(np.int64).tolist()
+        assert np.array_equal(s.sigmas.numpy(), np.append(x, 0).astype(np.float32))
+
+
+def test_schedule_takes_array_shifts_and_refuses_float_counts():
+    s = _sched(4, 5.0)
+    want = s.timesteps.tolist()
+    for shift in (np.array(5.0), np.float64(5.0), 5):
+        s.set_timesteps(4, shift=shift)
+        assert s.timesteps.tolist() == want
+    shift = np.array(3.0)
+    s.set_timesteps(4, shift=shift)
+    shift[()] = 5.0                                       # an array is read at each call, not remembered by its identity
+    s.set_timesteps(4, shift=shift)
+    assert s.timesteps.tolist() == want
+    with pytest.raises(TypeError):                        # as numpy.linspace refuses it, also behind a call with 4
+        s.set_timesteps(4.0, shift=5.0)
