@@ -133,10 +133,15 @@ __device__ __forceinline__ float ex2(float x) {
 }
 
 // three-input maximum (one instruction on sm_100) and packed two-lane fp32 arithmetic: they halve
-// the instruction count of the row maximum, the score scaling and the row sum
+// the instruction count of the row maximum, the score scaling and the row sum.  The maxima pass a NaN on (see row_max).
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+__device__ __forceinline__ float fmax2(float a, float b) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
   return d;
 }
 __device__ __forceinline__ void fma2(float& d0, float& d1, float a0, float a1, float b, float c) {
@@ -156,7 +161,8 @@ __device__ __forceinline__ void add2(float& d0, float& d1, float a0, float a1) {
 
 // exp2 of two values on the FMA pipe, for a share of the scores: floor by a round-down add of 1.5 * 2^23, a quartic for
 // 2^frac on [0, 1) (equal-ripple fit of the relative error with the constant term fixed at 1, by linear programming: 3e-6,
-// a thousandth of the bf16 rounding of P; the cubic of the same kind has 8.6e-5), exponent added as an integer.
+// a thousandth of the bf16 rounding of P; the cubic of the same kind has 8.6e-5), exponent added as an integer.  The clamp takes
+// a NaN for -125: the caller's row maximum has to carry it.
 __device__ __forceinline__ F2 ex2_poly2(F2 x) {
   x.x = fmaxf(x.x, -125.f);
   x.y = fmaxf(x.y, -125.f);
@@ -178,12 +184,13 @@ __device__ __forceinline__ F2 ex2_poly2(F2 x) {
 // 368: the quarter leaves the FMA pipe and the issue slots more room at the same time within the spread of runs.)
 __host__ __device__ constexpr bool poly_pair(int p) { return p % 4 == 1; }
 
-// Maximum of a row's scores: independent chains of three-input maxima.
+// Maximum of a row's scores: independent chains of three-input maxima.  NaN if a score is NaN, whatever its column: the FMA-pipe
+// exponential would lose it.
 __device__ __forceinline__ float row_max(const uint32_t (&sr)[4][32]) {
   constexpr int kChains = 8;
   float mx[kChains];
 #pragma unroll
-  for (int i = 0; i < kChains; ++i) mx[i] = fmaxf(__uint_as_float(sr[0][2 * i]), __uint_as_float(sr[0][2 * i + 1]));
+  for (int i = 0; i < kChains; ++i) mx[i] = fmax2(__uint_as_float(sr[0][2 * i]), __uint_as_float(sr[0][2 * i + 1]));
 #pragma unroll
   for (int i = 2 * kChains; i < 128; i += 2) {
     float& x = mx[(i >> 1) % kChains];
@@ -192,7 +199,7 @@ __device__ __forceinline__ float row_max(const uint32_t (&sr)[4][32]) {
 #pragma unroll
   for (int w = kChains / 2; w > 0; w >>= 1)
 #pragma unroll
-    for (int i = 0; i < w; ++i) mx[i] = fmaxf(mx[i], mx[i + w]);
+    for (int i = 0; i < w; ++i) mx[i] = fmax2(mx[i], mx[i + w]);
   return mx[0];
 }
 
@@ -481,7 +488,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (valid < kBK) mask_scores(sr, valid);
       const float mt = row_max(sr);
       // lazy rescale: keep the old offset unless this tile's maximum exceeds it by more than 2^8
-      const bool grow = (mt - m) * c > 8.f;           // also true for the first tile (m = -inf)
+      const bool grow = !((mt - m) * c <= 8.f);       // also true for the first tile (m = -inf) and for a NaN
       if (__any_sync(0xFFFFFFFFu, grow)) {
         if (j > 0) {
           // everything accumulated so far must have landed in O before it is rescaled
@@ -497,7 +504,9 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           m = mt;                                      // nothing accumulated yet
         }
       }
-      const float nmc = -m * c;
+      // A NaN or +inf score makes the row NaN, as inf - inf does in a softmax: NaN here reaches every exponential of the
+      // special-function unit, and with them the row sum.
+      const float nmc = __fmaf_rn(-m, c, m - m);
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
         uint32_t pk[16];

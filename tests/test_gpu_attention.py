@@ -364,3 +364,38 @@ def test_nvfp4kv_window_expansion_with_and_without_workspace(T, blocks, l_cur, s
     for n in (full, max(split, 16)):
         ws = torch.full((n,), 0xFF, dtype=torch.uint8, device="cuda")
         assert torch.equal(ops.attention_nvfp4kv(q, kq, vq, T, *cur, heads, key_splits=splits, workspace=ws), ref)
+
+
+def _softmax_attention(q, k, v, heads):
+    qh, kh, vh = (t.float().view(t.shape[0], heads, 128).transpose(0, 1) for t in (q, k, v))
+    return (torch.softmax(qh @ kh.transpose(1, 2) * 128 ** -0.5, -1) @ vh).transpose(0, 1).reshape(q.shape[0], heads * 128)
+
+
+@pytest.mark.parametrize("splits", [1, 2])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_attention_non_finite_key_reaches_the_output(bad, splits):
+    """One key with a NaN or an infinity, at every column position modulo 8 (two of eight take the FMA-pipe exponential) and in the
+    first, a middle and the ragged last key tile: the rows whose softmax is NaN are NaN, the others are as without it."""
+    heads, lq, lk = 2, 150, 300
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v = (torch.randn(n, heads * 128, generator=g, device="cuda").bfloat16() for n in (lq, lk, lk))
+    for key in [*range(8), 131, 138, 290, 299]:
+        kb = k.clone()
+        kb[key, 128 + 7] = bad                            # second head only
+        ref = _softmax_attention(q, kb, v, heads)
+        out = ops.attention_bf16(q, kb, v, heads, key_splits=splits).float()
+        assert torch.equal(out.isnan(), ref.isnan()), key
+        assert bool(ref[:, 128:].isnan().any()) and not bool(ref[:, :128].isnan().any())
+        ok = ~ref.isnan()
+        assert float((out[ok] - ref[ok]).norm() / ref[ok].norm()) < 1e-2
+
+
+def test_attention_non_finite_query_stays_in_its_row():
+    heads, lq, lk = 2, 300, 200
+    g = torch.Generator(device="cuda").manual_seed(6)
+    q, k, v = (torch.randn(n, heads * 128, generator=g, device="cuda").bfloat16() for n in (lq, lk, lk))
+    q[170, 3] = float("nan")
+    out = ops.attention_bf16(q, k, v, heads)
+    want = torch.zeros(lq, heads * 128, dtype=torch.bool, device="cuda")
+    want[170, :128] = True
+    assert torch.equal(out.isnan(), want)
