@@ -551,7 +551,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 // 0 with uniform splits).  L2 / launch bound: 9 us for the 116 cut items of the shape above (18 us with one row per warp and a
 // warp for every row of the output).
 constexpr int kCombineRows = 4;
-__global__ void __launch_bounds__(256) attention_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
+__global__ void __launch_bounds__(256) attention_combine_kernel(const float* part_o, const float* part_ml,
                                                                 int nsplit, int64_t Lq, int heads, float scale_log2,
                                                                 uint16_t* __restrict__ out, int64_t ldo, float* __restrict__ out_amax,
                                                                 int first_item, int q_tiles) {
@@ -573,16 +573,16 @@ __global__ void __launch_bounds__(256) attention_combine_kernel(const float* __r
   for (int z = 0; z < nsplit; ++z)
 #pragma unroll
     for (int r = 0; r < kCombineRows; ++r)
-      if (row0 + r < Lq) mmax[r] = fmaxf(mmax[r], __ldg(part_ml + (z * stride + (row0 + r) * heads + head) * 2));
+      if (row0 + r < Lq) mmax[r] = fmaxf(mmax[r], ld_global(part_ml + (z * stride + (row0 + r) * heads + head) * 2));
 #pragma unroll 2
   for (int z = 0; z < nsplit; ++z)
 #pragma unroll
     for (int r = 0; r < kCombineRows; ++r) {
       if (row0 + r >= Lq) continue;
       const int64_t unit = z * stride + (row0 + r) * heads + head;
-      const float2 ml = __ldg(reinterpret_cast<const float2*>(part_ml + unit * 2));
+      const float2 ml = ld_global(reinterpret_cast<const float2*>(part_ml + unit * 2));
       const float w = exp2f((ml.x - mmax[r]) * scale_log2);
-      const float4 o = __ldg(reinterpret_cast<const float4*>(part_o + unit * kD) + lane);
+      const float4 o = ld_global(reinterpret_cast<const float4*>(part_o + unit * kD) + lane);
       acc[r].x = __fmaf_rn(w, o.x, acc[r].x);
       acc[r].y = __fmaf_rn(w, o.y, acc[r].y);
       acc[r].z = __fmaf_rn(w, o.z, acc[r].z);

@@ -131,6 +131,12 @@ __device__ __forceinline__ void pdl_begin() {
   pdl_wait();
 }
 
+// Every load from global memory is an ordinary one.  A kernel's lifetime begins while its predecessor still writes (see launch_k), so
+// the read-only path (__ldg, or a const __restrict__ kernel parameter that the compiler turns into it) is not open: it asks for data
+// that nobody writes during the kernel's lifetime, and an invariant load may be moved above pdl_wait.
+template <typename T>
+__device__ __forceinline__ T ld_global(const T* p) { return *p; }
+
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 

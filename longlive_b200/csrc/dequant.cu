@@ -104,8 +104,8 @@ __device__ __forceinline__ float global_scale(int rounding, float amax, float de
 // rows x cols logical matrix; codes row stride = cols_padded/2 bytes; scales swizzled with
 // cols_padded/16 scale columns.
 template <typename T, int ROUNDING>
-__global__ void __launch_bounds__(256) dequant_matrix_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ sf,
-                                                             const float* __restrict__ amax_ptr, int64_t rows, int64_t cols,
+__global__ void __launch_bounds__(256) dequant_matrix_kernel(const uint8_t* codes, const uint8_t* sf,
+                                                             const float* amax_ptr, int64_t rows, int64_t cols,
                                                              int64_t cols_padded, float denom, T* __restrict__ out, int64_t ldo) {
   pdl_begin();
   const int64_t groups_per_row = cols >> 4;
@@ -114,8 +114,8 @@ __global__ void __launch_bounds__(256) dequant_matrix_kernel(const uint8_t* __re
   const float g = global_scale(ROUNDING, amax, denom);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = i / groups_per_row, c = i - r * groups_per_row;
-    const uint2 p = __ldg(reinterpret_cast<const uint2*>(codes + r * (cols_padded >> 1) + c * 8));
-    const float s = e4m3_to_float(__ldg(sf + sf_offset(r, c, cols_padded >> 4)));
+    const uint2 p = ld_global(reinterpret_cast<const uint2*>(codes + r * (cols_padded >> 1) + c * 8));
+    const float s = e4m3_to_float(ld_global(sf + sf_offset(r, c, cols_padded >> 4)));
     float v[16];
     decode16<ROUNDING>(p, s, amax, g, denom, v);
     store16<T>(out + r * ldo + c * 16, v);
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(256) dequant_kv_kernel(const __grid_constant__
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
       const int64_t r = i / vecs;
       const int c = (int)(i - r * vecs);
-      reinterpret_cast<uint4*>(copies.dst[m])[i] = __ldg(reinterpret_cast<const uint4*>(copies.src[m] + r * copies.ld[m]) + c);
+      reinterpret_cast<uint4*>(copies.dst[m])[i] = ld_global(reinterpret_cast<const uint4*>(copies.src[m] + r * copies.ld[m]) + c);
     }
     return;
   }
@@ -156,11 +156,11 @@ __global__ void __launch_bounds__(256) dequant_kv_kernel(const __grid_constant__
     const int64_t r = r0 + 16 * k;
     w[k] = sb[k] = 0u;
     if (r < rows) {
-      w[k] = __ldg(codes + r * 16 + c);
-      sb[k] = __ldg(sf + sf_offset(r, c >> 1, 8));
+      w[k] = ld_global(codes + r * 16 + c);
+      sb[k] = ld_global(sf + sf_offset(r, c >> 1, 8));
     }
   }
-  const float amax = __ldg(tab.amax[b]);
+  const float amax = ld_global(tab.amax[b]);
   const float g = global_scale(ROUNDING, amax, denom);
   T* out = (T*)tab.out[b];
 #pragma unroll

@@ -97,8 +97,8 @@ __device__ __forceinline__ void drain_chunk(const uint32_t (&r)[2][32], float al
 // swizzled staging buffer `buf` (32 rows x 128 bytes; with a residual the buffer holds the residual
 // tile on entry).  grow: this row's gate vector or nullptr.
 template <int EPI>
-__device__ __forceinline__ void epilogue_packed(const uint32_t (&pk)[32], const uint16_t* __restrict__ bias,
-                                                const uint16_t* __restrict__ grow, int64_t col, uint8_t* buf, int lane,
+__device__ __forceinline__ void epilogue_packed(const uint32_t (&pk)[32], const uint16_t* bias,
+                                                const uint16_t* grow, int64_t col, uint8_t* buf, int lane,
                                                 bool want_amax, bool row_ok, uint32_t& local_amax, const QuantOut* qo = nullptr,
                                                 bool store_bf16 = true) {
   constexpr bool has_res = (EPI & kEpiRes) != 0;
@@ -115,7 +115,7 @@ __device__ __forceinline__ void epilogue_packed(const uint32_t (&pk)[32], const 
 #pragma unroll
       for (int e = 0; e < 4; ++e) y[e] = unpack2(pk[v8 * 4 + e]);
       if (EPI & kEpiBias) {
-        const uint4 bv = __ldg(reinterpret_cast<const uint4*>(bias + col + v8 * 8));
+        const uint4 bv = ld_global(reinterpret_cast<const uint4*>(bias + col + v8 * 8));
         const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -134,7 +134,7 @@ __device__ __forceinline__ void epilogue_packed(const uint32_t (&pk)[32], const 
         const uint4 rv = *slot;
         const uint32_t rw[4] = {rv.x, rv.y, rv.z, rv.w};
         if (grow) {
-          const uint4 gv = __ldg(reinterpret_cast<const uint4*>(grow + col + v8 * 8));
+          const uint4 gv = ld_global(reinterpret_cast<const uint4*>(grow + col + v8 * 8));
           const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
 #pragma unroll
           for (int e = 0; e < 4; ++e) {

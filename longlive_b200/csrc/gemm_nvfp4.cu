@@ -210,15 +210,15 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     const int q = warp & 3;                           // TMEM lane quarter this warp may access
     const int half = warp >= 6 ? 1 : 0;               // which of the quarter's two warps this is
     float alpha0, alpha1 = 0.f, alpha2 = 0.f;           // per weight group (one group unless p.group_cols)
-    if (p.epi.alpha) alpha0 = __ldg(p.epi.alpha);
-    else alpha0 = __fdiv_rn(__fmul_rn(__ldg(p.a_amax), __ldg(p.b_amax)), p.alpha_denom);
+    if (p.epi.alpha) alpha0 = ld_global(p.epi.alpha);
+    else alpha0 = __fdiv_rn(__fmul_rn(ld_global(p.a_amax), ld_global(p.b_amax)), p.alpha_denom);
     if (p.group_cols) {
-      alpha1 = __fdiv_rn(__fmul_rn(__ldg(p.a_amax), __ldg(p.b_amax + 1)), p.alpha_denom);
-      if (p.N >= 3 * p.group_cols) alpha2 = __fdiv_rn(__fmul_rn(__ldg(p.a_amax), __ldg(p.b_amax + 2)), p.alpha_denom);
+      alpha1 = __fdiv_rn(__fmul_rn(ld_global(p.a_amax), ld_global(p.b_amax + 1)), p.alpha_denom);
+      if (p.N >= 3 * p.group_cols) alpha2 = __fdiv_rn(__fmul_rn(ld_global(p.a_amax), ld_global(p.b_amax + 2)), p.alpha_denom);
     }
     float amax0 = 0.f, amax1 = 0.f, amax2 = 0.f;
     quant::QuantConsts qconsts = {};
-    if constexpr ((EPI & kEpiQuant) != 0) qconsts = quant::make_consts<LLNV_RULE_MSE>(__ldg(p.q_amax));
+    if constexpr ((EPI & kEpiQuant) != 0) qconsts = quant::make_consts<LLNV_RULE_MSE>(ld_global(p.q_amax));
     const uint16_t* bias = reinterpret_cast<const uint16_t*>(p.epi.bias);
     constexpr bool has_res = (EPI & kEpiRes) != 0;
     const uint16_t* gate = reinterpret_cast<const uint16_t*>(p.epi.gate);

@@ -193,8 +193,8 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     const int q = warp & 3;                             // TMEM lane quarter this warp may access
     const int h = warp >= 6 ? 1 : 0;                    // column half of every tile this warp finishes
     float alpha;
-    if (p.epi.alpha) alpha = __ldg(p.epi.alpha);
-    else alpha = __fdiv_rn(__fmul_rn(__ldg(p.a_amax), __ldg(p.b_amax)), p.alpha_denom);
+    if (p.epi.alpha) alpha = ld_global(p.epi.alpha);
+    else alpha = __fdiv_rn(__fmul_rn(ld_global(p.a_amax), ld_global(p.b_amax)), p.alpha_denom);
     const uint16_t* bias = reinterpret_cast<const uint16_t*>(p.epi.bias);
     constexpr bool has_res = (EPI & kEpiRes) != 0;
     const uint16_t* gate = reinterpret_cast<const uint16_t*>(p.epi.gate);

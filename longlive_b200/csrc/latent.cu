@@ -18,7 +18,7 @@ namespace llnv {
 namespace {
 
 template <bool TO_TOKENS>
-__global__ void __launch_bounds__(256) latent_tokens_kernel(uint16_t* __restrict__ tokens, int64_t ldt, uint16_t* __restrict__ latent,
+__global__ void __launch_bounds__(256) latent_tokens_kernel(uint16_t* tokens, int64_t ldt, uint16_t* latent,
                                                             int64_t stride_c, int64_t stride_f, int C, int h, int w) {
   pdl_begin();
   extern __shared__ uint32_t sm[];                            // [w][2C + 1] words: (kw = 0, kw = 1) pairs

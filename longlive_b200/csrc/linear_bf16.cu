@@ -162,8 +162,8 @@ linear_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             const int cc = v8 * 8 + 2 * e;
             float y0 = __uint_as_float(r[cc >> 5][cc & 31]), y1 = __uint_as_float(r[(cc + 1) >> 5][(cc + 1) & 31]);
             if (p.bias) {
-              if (col + cc < p.N) y0 += __uint_as_float((uint32_t)__ldg(p.bias + col + cc) << 16);
-              if (col + cc + 1 < p.N) y1 += __uint_as_float((uint32_t)__ldg(p.bias + col + cc + 1) << 16);
+              if (col + cc < p.N) y0 += __uint_as_float((uint32_t)ld_global(p.bias + col + cc) << 16);
+              if (col + cc + 1 < p.N) y1 += __uint_as_float((uint32_t)ld_global(p.bias + col + cc + 1) << 16);
             }
             if (p.act) {
               round_bf16x2(y0, y1);

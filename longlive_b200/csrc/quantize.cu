@@ -46,7 +46,7 @@ using namespace quant;
 // divided into row and column.
 constexpr int kAmaxLoads = 8;
 template <bool ROWS>
-__device__ __forceinline__ uint32_t cta_amax_bits(const uint16_t* __restrict__ x, int64_t M, int64_t K, int64_t ldx, unsigned first,
+__device__ __forceinline__ uint32_t cta_amax_bits(const uint16_t* x, int64_t M, int64_t K, int64_t ldx, unsigned first,
                                                   unsigned stride) {
   const int64_t vec_per_row = K >> 3;
   const int64_t total = M * vec_per_row;
@@ -59,7 +59,7 @@ __device__ __forceinline__ uint32_t cta_amax_bits(const uint16_t* __restrict__ x
       v[j] = make_uint4(0u, 0u, 0u, 0u);
       if (i < total) {
         const int64_t r = ROWS ? i / vec_per_row : 0;
-        v[j] = __ldg(reinterpret_cast<const uint4*>(x + r * ldx) + (i - r * vec_per_row));
+        v[j] = ld_global(reinterpret_cast<const uint4*>(x + r * ldx) + (i - r * vec_per_row));
       }
     }
 #pragma unroll
@@ -80,7 +80,7 @@ __device__ __forceinline__ uint32_t cta_amax_bits(const uint16_t* __restrict__ x
 }
 
 template <bool F16, bool ROWS>
-__global__ void __launch_bounds__(256) amax_16bit_kernel(const uint16_t* __restrict__ x, int64_t M, int64_t K,
+__global__ void __launch_bounds__(256) amax_16bit_kernel(const uint16_t* x, int64_t M, int64_t K,
                                                          int64_t ldx, float* __restrict__ amax) {
   pdl_begin();
   const uint32_t mm = cta_amax_bits<ROWS>(x, M, K, ldx, blockIdx.x, gridDim.x);
@@ -146,11 +146,11 @@ __device__ __forceinline__ uint32_t ln_pair(uint32_t xw, uint32_t aw, uint32_t b
 template <int MODE>
 __device__ __forceinline__ void transform_block(uint32_t (&w)[8], const Prologue& pr, int64_t row, int64_t col) {
   if (MODE == kPlain || MODE == kPlainAmax) return;
-  const float mean = __ldg(pr.row_stats + 2 * row), rstd = __ldg(pr.row_stats + 2 * row + 1);
+  const float mean = ld_global(pr.row_stats + 2 * row), rstd = ld_global(pr.row_stats + 2 * row + 1);
   const int64_t prow = MODE == kAdaLN ? ((row + pr.row_offset) / pr.frame_rows) * pr.stride : 0;
   const uint4* a4 = reinterpret_cast<const uint4*>(pr.p0 + prow + col);
   const uint4* b4 = reinterpret_cast<const uint4*>(pr.p1 + prow + col);
-  const uint4 a0 = __ldg(a4), a1 = __ldg(a4 + 1), b0 = __ldg(b4), b1 = __ldg(b4 + 1);
+  const uint4 a0 = ld_global(a4), a1 = ld_global(a4 + 1), b0 = ld_global(b4), b1 = ld_global(b4 + 1);
   const uint32_t aw[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
   const uint32_t bw[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
   const F2 mean2 = f2_splat(mean), rstd2 = f2_splat(rstd);
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(256) quantize_nvfp4_kernel(const uint16_t* x, 
   auto load_block = [&](int i, uint32_t (&w)[8]) {
     if (32 * i < rows_left) {
       const uint4* p = reinterpret_cast<const uint4*>(xp);
-      const uint4 a = __ldg(p), b = __ldg(p + 1);
+      const uint4 a = ld_global(p), b = ld_global(p + 1);
       w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
       w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
     } else {
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(256) quantize_nvfp4_kernel(const uint16_t* x, 
 // WPR warps share one row (each takes C / WPR channels): with one warp per row a chunk of 2640
 // tokens is only 2640 warps and the kernel is bound by the latency of each warp's dependent steps.
 template <int MODE, int WPR>
-__global__ void __launch_bounds__(256, WPR > 1 ? 8 : 1) ln_stats_amax_kernel(const uint16_t* __restrict__ x, int64_t M, int64_t C, int64_t ldx,
+__global__ void __launch_bounds__(256, WPR > 1 ? 8 : 1) ln_stats_amax_kernel(const uint16_t* x, int64_t M, int64_t C, int64_t ldx,
                                                             float eps, Prologue pr, float* __restrict__ row_stats,
                                                             float* __restrict__ amax) {
   pdl_begin();
@@ -319,11 +319,11 @@ __global__ void __launch_bounds__(256, WPR > 1 ? 8 : 1) ln_stats_amax_kernel(con
   // fetches its few vectors of the two parameter rows itself, together with x)
   if (WPR == 1) {
     for (int i = threadIdx.x; i < nvec_all; i += blockDim.x) {
-      pa_sh[0][i] = __ldg(reinterpret_cast<const uint4*>(pr.p0 + f0 * pr.stride) + i);
-      pb_sh[0][i] = __ldg(reinterpret_cast<const uint4*>(pr.p1 + f0 * pr.stride) + i);
+      pa_sh[0][i] = ld_global(reinterpret_cast<const uint4*>(pr.p0 + f0 * pr.stride) + i);
+      pb_sh[0][i] = ld_global(reinterpret_cast<const uint4*>(pr.p1 + f0 * pr.stride) + i);
       if (f1 != f0) {
-        pa_sh[1][i] = __ldg(reinterpret_cast<const uint4*>(pr.p0 + f1 * pr.stride) + i);
-        pb_sh[1][i] = __ldg(reinterpret_cast<const uint4*>(pr.p1 + f1 * pr.stride) + i);
+        pa_sh[1][i] = ld_global(reinterpret_cast<const uint4*>(pr.p0 + f1 * pr.stride) + i);
+        pb_sh[1][i] = ld_global(reinterpret_cast<const uint4*>(pr.p1 + f1 * pr.stride) + i);
       }
     }
   }
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(256, WPR > 1 ? 8 : 1) ln_stats_amax_kernel(con
     for (int i = 0; i < kVec; ++i) {
       const int li = lane + 32 * i;
       if (li < pvec) {
-        v[i] = __ldg(reinterpret_cast<const uint4*>(x + row * ldx) + vbase + li);
+        v[i] = ld_global(reinterpret_cast<const uint4*>(x + row * ldx) + vbase + li);
         sum += bf16_lo(v[i].x) + bf16_hi(v[i].x) + bf16_lo(v[i].y) + bf16_hi(v[i].y) + bf16_lo(v[i].z) + bf16_hi(v[i].z) +
                bf16_lo(v[i].w) + bf16_hi(v[i].w);
       }
@@ -389,8 +389,8 @@ __global__ void __launch_bounds__(256, WPR > 1 ? 8 : 1) ln_stats_amax_kernel(con
       const int li = lane + 32 * i;
       if (li < pvec) {
         const int idx = vbase + li;
-        const uint4 a4 = WPR > 1 ? __ldg(reinterpret_cast<const uint4*>(pr.p0 + prow) + idx) : pa_sh[fsel][idx];
-        const uint4 b4 = WPR > 1 ? __ldg(reinterpret_cast<const uint4*>(pr.p1 + prow) + idx) : pb_sh[fsel][idx];
+        const uint4 a4 = WPR > 1 ? ld_global(reinterpret_cast<const uint4*>(pr.p0 + prow) + idx) : pa_sh[fsel][idx];
+        const uint4 b4 = WPR > 1 ? ld_global(reinterpret_cast<const uint4*>(pr.p1 + prow) + idx) : pb_sh[fsel][idx];
         const uint32_t ws[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
         const uint32_t aw[4] = {a4.x, a4.y, a4.z, a4.w};
         const uint32_t bw[4] = {b4.x, b4.y, b4.z, b4.w};

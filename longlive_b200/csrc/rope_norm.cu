@@ -44,12 +44,12 @@ struct RopeJobs {
 // device and the kernel would be bound by the latency of each warp's single pass.
 template <int WPR>
 __global__ void __launch_bounds__(256) rmsnorm_rope_kernel(const __grid_constant__ RopeJobs jobs, int64_t S, int64_t C, float eps,
-                                                           const float* __restrict__ cosv, const float* __restrict__ sinv,
+                                                           const float* cosv, const float* sinv,
                                                            int shard_vecs) {
   pdl_begin();
   const RopeJob& jb = jobs.job[blockIdx.y];
-  const uint16_t* __restrict__ x = jb.x;
-  const uint16_t* __restrict__ weight = jb.weight;
+  const uint16_t* x = jb.x;
+  const uint16_t* weight = jb.weight;
   const ShardOut& dst = jb.dst;
   const int64_t ldx = jb.ldx, ldo = jb.ldo, lds = jb.lds;
   const bool want_smooth = jb.want_smooth != 0;
@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(256) rmsnorm_rope_kernel(const __grid_constant
   const int pvec = nvec / WPR;               // vectors of this warp's part
   const int vbase = part * pvec;
   if (weight) {
-    for (int i = threadIdx.x; i < nvec; i += blockDim.x) w_sh[i] = __ldg(reinterpret_cast<const uint4*>(weight) + i);
+    for (int i = threadIdx.x; i < nvec; i += blockDim.x) w_sh[i] = ld_global(reinterpret_cast<const uint4*>(weight) + i);
   }
   // this lane needs the same 4 cos / 4 sin values in every step (pair index depends on lane only:
   // a part starts on a head boundary)
@@ -77,8 +77,8 @@ __global__ void __launch_bounds__(256) rmsnorm_rope_kernel(const __grid_constant
   if (row < S) {
     if (cosv) {
       const int pair0 = (lane & 15) * 4;
-      const float4 c4 = __ldg(reinterpret_cast<const float4*>(cosv + row * 64 + pair0));
-      const float4 s4 = __ldg(reinterpret_cast<const float4*>(sinv + row * 64 + pair0));
+      const float4 c4 = ld_global(reinterpret_cast<const float4*>(cosv + row * 64 + pair0));
+      const float4 s4 = ld_global(reinterpret_cast<const float4*>(sinv + row * 64 + pair0));
       cc[0] = c4.x; cc[1] = c4.y; cc[2] = c4.z; cc[3] = c4.w;
       sn[0] = s4.x; sn[1] = s4.y; sn[2] = s4.z; sn[3] = s4.w;
     }
@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(256) rmsnorm_rope_kernel(const __grid_constant
     for (int i = 0; i < kVec; ++i) {
       const int li = lane + 32 * i;
       if (li < pvec) {
-        v[i] = __ldg(reinterpret_cast<const uint4*>(x + row * ldx) + vbase + li);
+        v[i] = ld_global(reinterpret_cast<const uint4*>(x + row * ldx) + vbase + li);
         const uint32_t w4[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {

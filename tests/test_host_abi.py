@@ -106,3 +106,12 @@ def test_documented_python_seam_names_exist():
         assert hasattr(longlive_b200, name), name
     sched = longlive_b200.scheduler.FlowUniPCMultistepScheduler
     assert all(hasattr(sched, m) for m in ("set_timesteps", "step"))
+
+
+def test_kernels_read_global_memory_with_ordinary_loads():
+    """A kernel's lifetime begins while its predecessor writes (programmatic launches), so none reads through the read-only path: no
+    __ldg, no ld.global.nc, and no const __restrict__ parameter that the compiler could turn into one."""
+    src = os.path.join(ROOT, "longlive_b200", "csrc")
+    for name in sorted(os.listdir(src)):
+        code = re.sub(r"//.*", "", open(os.path.join(src, name)).read())
+        assert not re.search(r"__ldg\s*\(|ld\.global\.nc|const\s+[\w:]+\s*\*\s*__restrict__", code), name
