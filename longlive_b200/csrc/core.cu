@@ -59,24 +59,26 @@ void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 
 namespace {
 thread_local int g_amax_accumulate = 0;
-int g_pdl = -1;                        // -1: not decided yet (on, unless the environment has LLNV_PDL=0)
+std::atomic<int> g_pdl{-1};            // read by every thread that launches; -1: not decided yet (on, unless the environment has LLNV_PDL=0)
 }
 
 bool amax_accumulate(int which) { return (g_amax_accumulate & which) != 0; }
 
 bool pdl_enabled() {
-  if (g_pdl < 0) {
+  int on = g_pdl.load(std::memory_order_relaxed);
+  if (on < 0) {
     const char* e = getenv("LLNV_PDL");
-    g_pdl = (e && e[0] == '0') ? 0 : 1;
+    const int from_env = (e && e[0] == '0') ? 0 : 1;
+    on = g_pdl.compare_exchange_strong(on, from_env, std::memory_order_relaxed) ? from_env : on;      // or what llnv_set_pdl just set
   }
-  return g_pdl != 0;
+  return on != 0;
 }
 
 }  // namespace llnv
 
 extern "C" int llnv_set_pdl(int on) {
   const int before = llnv::pdl_enabled() ? 1 : 0;
-  llnv::g_pdl = on ? 1 : 0;
+  llnv::g_pdl.store(on ? 1 : 0, std::memory_order_relaxed);
   return before;
 }
 
