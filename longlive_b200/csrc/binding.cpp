@@ -5,6 +5,9 @@
 // (device context manager, stream lookup, a foreign call with 20 boxed arguments, torch.empty for every output), and a
 // module call on 17 rows spent 58 us on a device that was busy for 24 us.  Here the same work takes about 2 us per
 // operation.  Group (sequence-parallel) forms stay on ctypes: they are bound by the exchange.
+//
+// Every function runs without the interpreter lock, as a ctypes call does: a launch blocks while the launch queue is full, and a first
+// use loads kernels.  Only attention_nvfp4kv takes Python objects, which it unpacks before it lets the lock go.
 #include <Python.h>
 
 #include <ATen/ATen.h>
@@ -15,6 +18,7 @@
 #include <atomic>
 #include <optional>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "../../include/llnvfp4.h"
@@ -93,11 +97,11 @@ Quantized quantize_impl(Tensor x, int rule, OptTensor amax, OptTensor codes, Opt
   return q;
 }
 
-py::tuple quantize(const Tensor& x, int rule, OptTensor amax, OptTensor codes, OptTensor sf, std::optional<bool> amax_given) {
+std::tuple<Tensor, Tensor, Tensor> quantize(const Tensor& x, int rule, OptTensor amax, OptTensor codes, OptTensor sf, std::optional<bool> amax_given) {
   require_cuda(x, "x");
   const bool given = amax_given ? *amax_given : amax.has_value();
   Quantized q = quantize_impl(x, rule, amax, codes, sf, given);
-  return py::make_tuple(q.codes, q.sf, q.amax);
+  return {q.codes, q.sf, q.amax};
 }
 
 void quantize_pair(const Tensor& x0, const Tensor& x1, int rule, const Tensor& c0, const Tensor& s0, const Tensor& a0, const Tensor& c1,
@@ -111,7 +115,9 @@ void quantize_pair(const Tensor& x0, const Tensor& x1, int rule, const Tensor& c
                                  fptr(a1), given, call.stream));
 }
 
-py::tuple adaln_quantize(const Tensor& x, const Tensor& scale, const Tensor& shift, int frame_rows, int rule, double eps, bool add_one,
+using QuantizedAndY = std::tuple<OptTensor, OptTensor, OptTensor, OptTensor>;
+
+QuantizedAndY adaln_quantize(const Tensor& x, const Tensor& scale, const Tensor& shift, int frame_rows, int rule, double eps, bool add_one,
                          bool want_y, OptTensor codes, OptTensor sf, OptTensor amax, OptTensor row_stats, int64_t row_offset, int phase,
                          bool y_only) {
   require_cuda(x, "x");
@@ -134,10 +140,10 @@ py::tuple adaln_quantize(const Tensor& x, const Tensor& scale, const Tensor& shi
   if (want_y) y = empty(x, {m, c}, at::kBFloat16);
   check(llnv_adaln_quantize_nvfp4_ex(ptr(x), m, c, x.stride(0), ptr(scale), ptr(shift), scale.stride(0), frame_rows, (float)eps, add_one, rule,
                                      ptr(codes), ptr(sf), fptr(amax), ptr(y), c, fptr(row_stats), row_offset, phase, call.stream));
-  return py::make_tuple(codes, sf, amax, y);
+  return {codes, sf, amax, y};
 }
 
-py::tuple layernorm_quantize(const Tensor& x, const Tensor& weight, const Tensor& bias, int rule, double eps, bool want_y, OptTensor codes,
+QuantizedAndY layernorm_quantize(const Tensor& x, const Tensor& weight, const Tensor& bias, int rule, double eps, bool want_y, OptTensor codes,
                              OptTensor sf, OptTensor amax, OptTensor row_stats, int phase) {
   require_cuda(x, "x");
   if (!is_2d_bf16(x)) fail("layernorm_quantize_nvfp4 expects a 2-D bfloat16 tensor with unit column stride");
@@ -151,11 +157,11 @@ py::tuple layernorm_quantize(const Tensor& x, const Tensor& weight, const Tensor
   if (want_y) y = empty(x, {m, c}, at::kBFloat16);
   check(llnv_layernorm_quantize_nvfp4_ex(ptr(x), m, c, x.stride(0), ptr(weight), ptr(bias), (float)eps, rule, ptr(codes), ptr(sf), fptr(amax),
                                          ptr(y), c, fptr(row_stats), phase, call.stream));
-  return py::make_tuple(codes, sf, amax, y);
+  return {codes, sf, amax, y};
 }
 
 // ---- RMSNorm + RoPE -------------------------------------------------------------------------------
-py::tuple rmsnorm_rope(const Tensor& x, OptTensor weight, OptTensor cosv, OptTensor sinv, double eps, OptTensor out, OptTensor smooth,
+std::tuple<OptTensor, OptTensor, OptTensor> rmsnorm_rope(const Tensor& x, OptTensor weight, OptTensor cosv, OptTensor sinv, double eps, OptTensor out, OptTensor smooth,
                        bool want_smooth, OptTensor amax, bool want_amax, int shards) {
   require_cuda(x, "x");
   if (!is_2d_bf16(x)) fail("rmsnorm_rope expects a 2-D bfloat16 tensor with unit column stride");
@@ -173,7 +179,7 @@ py::tuple rmsnorm_rope(const Tensor& x, OptTensor weight, OptTensor cosv, OptTen
     fail("cos/sin must be contiguous float32 [S, 64]");
   check(llnv_rmsnorm_rope_ex(ptr(x), s, c, x.stride(0), ptr(weight), (float)eps, fptr(cosv), fptr(sinv), ptr(out), out->stride(-2), ptr(smooth),
                              smooth ? smooth->stride(-2) : 0, fptr(amax), shards, call.stream));
-  return py::make_tuple(out, smooth, amax);
+  return {out, smooth, amax};
 }
 
 using Ptrs = std::vector<uintptr_t>;
@@ -342,6 +348,7 @@ Tensor attention_nvfp4kv(const Tensor& q, const py::sequence& k_blocks, const py
   const int n = (int)k_blocks.size();
   if ((int)v_blocks.size() != n) fail("k_blocks and v_blocks must have the same length");
   const Blocks kb = gather_blocks(k_blocks, q, (int64_t)block_tokens * heads), vb = gather_blocks(v_blocks, q, (int64_t)block_tokens * heads);
+  const py::gil_scoped_release nogil;
   int64_t l_cur = 0;
   if (k_cur) {
     if (!is_heads_matrix(*k_cur, heads)) fail("k_cur must be bfloat16 [tokens, heads*128] with unit column stride");
@@ -475,22 +482,23 @@ uintptr_t current_stream(int device) { return reinterpret_cast<uintptr_t>(c10::c
 }  // namespace
 
 PYBIND11_MODULE(_native, m) {
-  m.def("quantize", &quantize);
-  m.def("quantize_pair", &quantize_pair);
-  m.def("adaln_quantize", &adaln_quantize);
-  m.def("layernorm_quantize", &layernorm_quantize);
-  m.def("rmsnorm_rope", &rmsnorm_rope);
-  m.def("rmsnorm_rope_qk", &rmsnorm_rope_qk);
-  m.def("gemm", &gemm);
-  m.def("gemm_grouped", &gemm_grouped);
-  m.def("linear_nvfp4", &linear_nvfp4);
-  m.def("attention_bf16", &attention_bf16);
-  m.def("attention_nvfp4kv", &attention_nvfp4kv);
-  m.def("dequantize", &dequantize);
-  m.def("kv_dequant", &kv_dequant);
-  m.def("linear_bf16", &linear_bf16);
-  m.def("patchify", &patchify);
-  m.def("unpatchify", &unpatchify);
-  m.def("unipc_step", &unipc_step);
-  m.def("current_stream", &current_stream);
+  using Unlocked = py::call_guard<py::gil_scoped_release>;
+  m.def("quantize", &quantize, Unlocked());
+  m.def("quantize_pair", &quantize_pair, Unlocked());
+  m.def("adaln_quantize", &adaln_quantize, Unlocked());
+  m.def("layernorm_quantize", &layernorm_quantize, Unlocked());
+  m.def("rmsnorm_rope", &rmsnorm_rope, Unlocked());
+  m.def("rmsnorm_rope_qk", &rmsnorm_rope_qk, Unlocked());
+  m.def("gemm", &gemm, Unlocked());
+  m.def("gemm_grouped", &gemm_grouped, Unlocked());
+  m.def("linear_nvfp4", &linear_nvfp4, Unlocked());
+  m.def("attention_bf16", &attention_bf16, Unlocked());
+  m.def("attention_nvfp4kv", &attention_nvfp4kv);       // lets the lock go itself
+  m.def("dequantize", &dequantize, Unlocked());
+  m.def("kv_dequant", &kv_dequant, Unlocked());
+  m.def("linear_bf16", &linear_bf16, Unlocked());
+  m.def("patchify", &patchify, Unlocked());
+  m.def("unpatchify", &unpatchify, Unlocked());
+  m.def("unipc_step", &unipc_step, Unlocked());
+  m.def("current_stream", &current_stream, Unlocked());
 }

@@ -158,3 +158,41 @@ def test_calls_from_two_threads(pdl):
     assert not errors, errors
     _same(want[0], got[0])
     _same(want[1], got[1])
+
+
+@pytest.mark.parametrize("op", ["quantize", "window"])
+def test_a_blocked_launch_leaves_other_threads_running(op):
+    """Behind half a second of device work the launch queue fills up and a launch blocks: meanwhile another Python thread goes on."""
+    import time
+    chain = Chain(1)
+    codes, sf, amax = ops.quantize_nvfp4(chain.x, 3)
+    if op == "quantize":
+        call = lambda: ops.quantize_nvfp4(chain.x, 3, amax, codes, sf)
+    else:
+        call = lambda: ops.attention_nvfp4kv(chain.x, *chain.blocks, chain.tokens, chain.x, chain.x, chain.heads, out=chain.out, key_splits=2,
+                                             workspace=chain.ws)
+    call()
+    torch.cuda.synchronize()
+    stop, gaps = threading.Event(), []
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.002)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+
+    ticker = threading.Thread(target=tick)
+    ticker.start()
+    torch.cuda._sleep(1_000_000_000)
+    longest = 0.0
+    for _ in range(3000):
+        t0 = time.perf_counter()
+        call()
+        longest = max(longest, time.perf_counter() - t0)
+    torch.cuda.synchronize()
+    stop.set()
+    ticker.join()
+    assert longest > 0.1, "the launch queue never filled"
+    assert max(gaps) < longest / 2
