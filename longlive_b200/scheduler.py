@@ -25,6 +25,9 @@ from . import _lib
 from .ops import _require_cuda
 
 
+_PLAIN = (int, float)
+
+
 def _lam(sigma: torch.Tensor) -> torch.Tensor:
     return torch.log(1 - sigma) - torch.log(sigma)
 
@@ -113,17 +116,19 @@ class FlowUniPCMultistepScheduler:
             shift = self.shift
         # The grid is a host table of a few numbers; a video sets the same one for every chunk.  The key holds everything the grid is
         # made of, and only plain numbers: their hash is their value (a tensor's is its identity), and 4 is not 4.0 to linspace.
-        key = (num_inference_steps, shift, self.sigma_max, self.sigma_min, self.num_train_timesteps)
-        if sigmas is not None or type(num_inference_steps) is not int or not all(type(v) in (int, float) for v in key):
-            key = None
-        grid = self._grids.get(key) if key is not None else None
+        high, low, scale = self.sigma_max, self.sigma_min, self.num_train_timesteps
+        key = grid = None
+        if (sigmas is None and type(num_inference_steps) is int and type(shift) in _PLAIN and type(high) in _PLAIN and type(low) in _PLAIN
+                and type(scale) in _PLAIN):
+            key = (num_inference_steps, shift, high, low, scale)
+            grid = self._grids.get(key)
         if grid is None:
             if sigmas is None:
-                sigmas = np.linspace(self.sigma_max, self.sigma_min, num_inference_steps + 1).copy()[:-1]
+                sigmas = np.linspace(high, low, num_inference_steps + 1).copy()[:-1]
             else:
                 sigmas = np.asarray(sigmas, dtype=np.float64)
             sigmas = shift * sigmas / (1 + (shift - 1) * sigmas)
-            host = (sigmas * self.num_train_timesteps).astype(np.int64)
+            host = (sigmas * scale).astype(np.int64)
             grid = (torch.from_numpy(np.concatenate([sigmas, [0]]).astype(np.float32)), torch.from_numpy(host), host.tolist())
             if key is not None:
                 if len(self._grids) >= 64:
