@@ -166,6 +166,7 @@ std::tuple<OptTensor, OptTensor, OptTensor> rmsnorm_rope(const Tensor& x, OptTen
   require_cuda(x, "x");
   if (!is_2d_bf16(x)) fail("rmsnorm_rope expects a 2-D bfloat16 tensor with unit column stride");
   const int64_t s = x.size(0), c = x.size(1);
+  if (shards < 1 || c % shards != 0) fail("rmsnorm_rope: " + std::to_string(c) + " channels do not divide into " + std::to_string(shards) + " shards");
   Call call(x);
   const std::vector<int64_t> shape = shards == 1 ? std::vector<int64_t>{s, c} : std::vector<int64_t>{shards, s, c / shards};
   if (!out) out = empty(x, shape, at::kBFloat16);
@@ -188,6 +189,7 @@ void* const* table(const Ptrs& p) { return reinterpret_cast<void* const*>(p.data
 void rmsnorm_rope_qk(const Tensor& xq, const Tensor& wq, const Ptrs& q, int64_t ldq, const Tensor& xk, const Tensor& wk, const Ptrs& k,
                      int64_t ldk, const std::optional<Ptrs>& ks, int64_t lds, OptTensor k_amax, const Tensor& cosv, const Tensor& sinv, double eps) {
   require_cuda(xq, "xq");
+  if (k.size() != q.size() || (ks && ks->size() != q.size())) fail("rmsnorm_rope_qk: one address per head shard for each output");
   Call call(xq);
   check(llnv_rmsnorm_rope_qk(ptr(xq), xq.stride(0), ptr(wq), table(q), ldq, ptr(xk), xk.stride(0), ptr(wk), table(k), ldk,
                              ks ? table(*ks) : nullptr, lds, fptr(k_amax), xq.size(0), xq.size(1), (float)eps, fptr(cosv), fptr(sinv),

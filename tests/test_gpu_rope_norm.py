@@ -101,3 +101,19 @@ def test_qk_prologue_in_one_launch():
     am = torch.zeros(1, dtype=torch.float32, device="cuda")
     ops.rmsnorm_rope_qk(xq, wq, [q.data_ptr()], c, xk, wk, [k.data_ptr()], c, [ks.data_ptr()], c, am, cos, sin, 1e-6)
     assert torch.equal(q, q_ref) and torch.equal(k, k_ref) and torch.equal(ks, ks_ref) and torch.equal(am, am_ref)
+
+
+@pytest.mark.parametrize("shards", [0, -1, 3])
+def test_prologue_refuses_shards_that_do_not_divide(shards):
+    """An error, not an integer division by zero in native code."""
+    x = torch.zeros(4, 512, dtype=torch.bfloat16, device="cuda")
+    with pytest.raises(RuntimeError, match="shards"):
+        ops.rmsnorm_rope(x, shards=shards)
+
+
+def test_qk_prologue_refuses_tables_of_different_length():
+    x = torch.zeros(4, 512, dtype=torch.bfloat16, device="cuda")
+    w, t = x[0].clone(), torch.zeros(4, 64, device="cuda")
+    p = [x.data_ptr()]
+    with pytest.raises(RuntimeError, match="one address"):
+        ops.rmsnorm_rope_qk(x, w, p * 2, 256, x, w, p, 256, None, 0, None, t, t, 1e-6)
