@@ -16,6 +16,7 @@
 #include <torch/extension.h>
 
 #include <atomic>
+#include <initializer_list>
 #include <optional>
 #include <string>
 #include <tuple>
@@ -197,12 +198,28 @@ void rmsnorm_rope_qk(const Tensor& xq, const Tensor& wq, const Ptrs& q, int64_t 
 }
 
 // ---- GEMM -----------------------------------------------------------------------------------------
+void same_device(const Tensor& like, std::initializer_list<const Tensor*> ts) {
+  for (const Tensor* t : ts)
+    if (t->device() != like.device()) fail("operands of a GEMM must be on one device (" + like.device().str() + " and " + t->device().str() + ")");
+}
+
+// The bias as the epilogue reads it, n packed bf16 values: a module in another precision has a bias of that precision.
+OptTensor packed_bias(const OptTensor& bias, int64_t n, const Tensor& like) {
+  if (!bias) return std::nullopt;
+  same_device(like, {&*bias});
+  if (bias->numel() < n) fail("bias holds " + std::to_string(bias->numel()) + " values, " + std::to_string(n) + " are needed");
+  if (bias->scalar_type() == at::kBFloat16 && bias->is_contiguous()) return bias;
+  return bias->to(at::kBFloat16).contiguous();
+}
+
 OptTensor gemm(const Tensor& a_codes, const Tensor& a_sf, OptTensor a_amax, int a_rule, const Tensor& b_codes, const Tensor& b_sf,
                OptTensor b_amax, int b_rule, int64_t m, int64_t n, int64_t k, OptTensor out, OptTensor alpha, OptTensor bias, int act,
                OptTensor residual, OptTensor gate, int frame_rows, OptTensor out_amax, int row_offset, int tile, OptTensor q_codes,
                OptTensor q_sf, OptTensor q_amax, bool store_out) {
   require_cuda(a_codes, "a_codes");
+  same_device(a_codes, {&a_sf, &b_codes, &b_sf});
   Call call(a_codes);
+  bias = packed_bias(bias, n, a_codes);
   if (!q_codes && !store_out) bad_value("store_out=False needs requant buffers");
   if (!out && store_out) out = empty(a_codes, {m, n}, at::kBFloat16);
   llnv_epilogue_t epi = {};
@@ -239,7 +256,9 @@ void gemm_grouped(const Tensor& a_codes, const Tensor& a_sf, const Tensor& a_ama
                   const Tensor& b_amax, int b_rule, int64_t m, int64_t n_each, int64_t k, const std::vector<Tensor>& outs, OptTensor bias, int act,
                   const std::optional<std::vector<OptTensor>>& out_amax) {
   require_cuda(a_codes, "a_codes");
+  same_device(a_codes, {&a_sf, &b_codes, &b_sf, &b_amax});
   Call call(a_codes);
+  bias = packed_bias(bias, n_each * (int64_t)outs.size(), a_codes);
   llnv_epilogue_t epi = {};
   epi.bias = ptr(bias);
   epi.act = act;
@@ -262,13 +281,14 @@ Tensor linear_nvfp4(const Tensor& input, int a_rule, const Tensor& w_codes, cons
                     int64_t n_pad, int64_t k, OptTensor bias) {
   const Tensor x = input.dim() == 2 ? input : input.reshape({-1, k});
   const int64_t m = x.size(0);
+  same_device(x, {&w_codes, &w_sf, &w_amax});
   Quantized q = quantize_impl(x, a_rule, std::nullopt, std::nullopt, std::nullopt, false);
   Call call(x);
   Tensor out = empty(x, {m, n_pad}, at::kBFloat16);
-  Tensor b;
-  if (bias) b = bias->numel() == n_pad ? *bias : at::constant_pad_nd(*bias, {0, n_pad - bias->numel()});
+  if (bias && bias->numel() != n_pad) bias = at::constant_pad_nd(*bias, {0, n_pad - bias->numel()});
+  bias = packed_bias(bias, n_pad, x);
   llnv_epilogue_t epi = {};
-  if (b.defined()) epi.bias = ptr(b);
+  epi.bias = ptr(bias);
   check(llnv_gemm_nvfp4(ptr(q.codes), ptr(q.sf), fptr(q.amax), a_rule, ptr(w_codes), ptr(w_sf), fptr(w_amax), w_rule, m, n_pad, k, &epi,
                         ptr(out), n_pad, call.stream));
   if (n != n_pad) out = out.narrow(1, 0, n);

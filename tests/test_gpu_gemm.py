@@ -366,3 +366,52 @@ def test_gemm_epilogue_chunks_over_many_tiles(m, n, k, tile):
     ok = ~ref.isnan()
     assert int((~ok).sum()) == 1 and torch.equal(y[ok], ref[ok]) and bool(y[m // 2, 5].isnan())
     assert float(amax.item()) == float(ref[ok].float().abs().max().item())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("n", [256, 200])
+def test_bias_of_another_precision(n, dtype):
+    """A bias that is not packed bf16 (of an fp16 module, an fp32 one, a strided view) is rounded to bf16, in the module, in the matrix
+    product and in the single and grouped GEMM; too short a bias or a weight on the host is an error."""
+    g = torch.Generator().manual_seed(n)
+    x = util.config_activation(33, 512, seed=2).cuda()
+    w = util.config_weight(n, 512).cuda()
+    bias = torch.randn(n, generator=g).to(dtype).cuda()
+    for b in (bias, torch.stack([bias, bias + 1], 1)[:, 0]):
+        mods = []
+        for value in (b, b.bfloat16().contiguous()):
+            m = torch.nn.Sequential(torch.nn.Linear(512, n, bias=True, device="cuda", dtype=torch.bfloat16))
+            with torch.no_grad():
+                m[0].weight.copy_(w)
+            m[0].bias = torch.nn.Parameter(value, requires_grad=False)
+            L.quantize_model(m, L.ModelQuantizationConfig())
+            m[0].materialize()
+            mods.append(m[0])
+        assert mods[0].bias.dtype == dtype
+        assert torch.equal(mods[0](x), mods[1](x))
+        xq, wq = L.quantize_to_fp4(x), mods[0].quantized_weight()
+        assert torch.equal(L.fp4_matmul(xq, wq, bias=b), mods[1](x))
+    if n == 256:
+        args = (xq.values, xq.scale_factors, xq.amax, 3, wq.values, wq.scale_factors, wq.amax, 3)
+        outs = [torch.empty(33, 128, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+        ops.gemm_nvfp4_grouped(*args[:6], wq.amax.repeat(2), 3, 33, 128, 512, outs, bias=bias)
+        assert torch.equal(torch.cat(outs, 1), ops.gemm_nvfp4(*args, 33, n, 512, bias=bias.bfloat16()))
+        with pytest.raises(RuntimeError, match="bias"):
+            ops.gemm_nvfp4(*args, 33, n, 512, bias=bias[:128].contiguous())
+    cpu = torch.nn.Sequential(torch.nn.Linear(512, n, device="cuda", dtype=torch.bfloat16))
+    L.quantize_model_with_filter(cpu, materialize_for_inference=True, verbose=False)
+    with pytest.raises(RuntimeError, match="one device"):
+        cpu[0].cpu()(x)
+
+
+def test_fp16_linear_with_bias():
+    """A half-precision nn.Linear converted as it is: fp16 activations, weight and bias."""
+    lin = torch.nn.Linear(512, 256, device="cuda", dtype=torch.float16)
+    x = util.config_activation(20, 512, seed=3).half().cuda()
+    m = torch.nn.Sequential(lin)
+    bias = lin.bias.detach().clone()
+    L.quantize_model(m, L.ModelQuantizationConfig())
+    m[0].materialize()
+    got = m(x)
+    no_bias = L.fp4_matmul(L.quantize_to_fp4(x), m[0].quantized_weight())
+    assert torch.equal(got, no_bias + bias.bfloat16())
