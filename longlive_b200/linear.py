@@ -199,6 +199,7 @@ class FourOverSixLinear(nn.Linear):
         cfg = self.config
         if (input.is_cuda and input.dtype in _ACTIVATIONS and cfg.dtype is DataType.nvfp4 and cfg.output_dtype is DataType.bfloat16
                 and cfg.quantize_backend in _QUANTIZE_BACKENDS and cfg.matmul_backend in _MATMUL_BACKENDS
+                and type(cfg.activation_scale_rule) is ScaleRule      # a rule assigned by name is resolved below
                 and input.shape[-1] == w.original_shape[1] == w.padded_shape[1] and w.padded_shape[1] % 256 == 0 and input.numel()):
             # the same three steps as below in one native call: at few tokens the module call is bound by the host
             return _lib.native().linear_nvfp4(input, cfg.activation_scale_rule.cuda_id(), w.values, w.scale_factors, w.amax,

@@ -43,6 +43,15 @@ def _check(rc: int) -> None:
         raise RuntimeError(f"llnvfp4 error {rc}: {msg}")
 
 
+def _seq(x):
+    """The binding takes lists and tuples; any other iterable (a dictionary's values, a stacked tensor) is listed first."""
+    return x if x is None or type(x) in (list, tuple) else list(x)
+
+
+def _opt_int(x):
+    return None if x is None else int(x)
+
+
 def padded_rows(m: int) -> int:
     return (m + 127) // 128 * 128
 
@@ -121,7 +130,7 @@ def adaln_quantize_nvfp4(x, scale, shift, frame_rows, rule_id, eps=1e-6, add_one
     over the group inside the quantize kernel (``llnv_adaln_quantize_nvfp4_group``)."""
     if group is None:
         return _lib.native().adaln_quantize(x, scale, shift, int(frame_rows), rule_id, eps, add_one, want_y, codes, sf, amax, row_stats,
-                                            row_offset, phase, y_only)
+                                            int(row_offset), int(phase), y_only)
     _require_cuda(x, "x")
     if x.dim() != 2 or x.dtype != torch.bfloat16 or x.stride(1) != 1:
         raise RuntimeError("adaln_quantize_nvfp4 expects a 2-D bfloat16 tensor with unit column stride")
@@ -146,7 +155,7 @@ def layernorm_quantize_nvfp4(x, weight, bias, rule_id, eps=1e-6, *, want_y=False
     """Affine LayerNorm fused with the NVFP4 quantize of its output.  Returns (codes, sf, amax, y or None).
     ``group`` (a ``sp.PeerArena``): the tensor amax is MAX-reduced over the group inside the quantize kernel."""
     if group is None:
-        return _lib.native().layernorm_quantize(x, weight, bias, rule_id, eps, want_y, codes, sf, amax, row_stats, phase)
+        return _lib.native().layernorm_quantize(x, weight, bias, rule_id, eps, want_y, codes, sf, amax, row_stats, int(phase))
     _require_cuda(x, "x")
     if x.dim() != 2 or x.dtype != torch.bfloat16 or x.stride(1) != 1:
         raise RuntimeError("layernorm_quantize_nvfp4 expects a 2-D bfloat16 tensor with unit column stride")
@@ -199,7 +208,7 @@ def rmsnorm_rope_scatter(x, weight, cos, sin, eps, out_ptrs, ldo, smooth_ptrs=No
 def rmsnorm_rope_qk(xq, wq, q_ptrs, ldq, xk, wk, k_ptrs, ldk, k_smooth_ptrs, lds, k_amax, cos, sin, eps):
     """The q and the k prologue of a block in one launch (``llnv_rmsnorm_rope_qk``); outputs are raw
     device addresses, one per head shard."""
-    _lib.native().rmsnorm_rope_qk(xq, wq, q_ptrs, ldq, xk, wk, k_ptrs, ldk, k_smooth_ptrs, lds, k_amax, cos, sin, eps)
+    _lib.native().rmsnorm_rope_qk(xq, wq, _seq(q_ptrs), ldq, xk, wk, _seq(k_ptrs), ldk, _seq(k_smooth_ptrs), lds, k_amax, cos, sin, eps)
 
 
 def scatter_2d(src, src_shard_bytes, dst_ptrs, dst_pitch, rows, row_bytes):
@@ -277,7 +286,7 @@ def attention_bf16(q, k, v, heads, scale=None, out=None, key_splits=None, out_am
     device, 1 unless the tiles alone leave most SMs idle).  ``out_amax`` (fp32 [1]) receives max |out|.
     ``workspace``: a uint8 tensor for the partial results of a split call (``attention_workspace_bytes``); allocated
     per call when omitted."""
-    return _lib.native().attention_bf16(q, k, v, heads, scale, out, key_splits, out_amax, workspace)
+    return _lib.native().attention_bf16(q, k, v, heads, scale, out, _opt_int(key_splits), out_amax, workspace)
 
 
 def attention_nvfp4kv(q, k_blocks, v_blocks, block_tokens, k_cur, v_cur, heads, scale=None, out=None, key_splits=None,
@@ -288,8 +297,8 @@ def attention_nvfp4kv(q, k_blocks, v_blocks, block_tokens, k_cur, v_cur, heads, 
     ``block_tokens * heads`` rows of 128 channels, token-major / head-minor).  ``k_cur`` / ``v_cur``: bf16
     [L_cur, heads*128] (or None when the window is the cache alone).  Result: bf16 [Lq, heads*128], equal bit
     for bit to dequantizing the blocks into a window and calling ``attention_bf16`` on it."""
-    return _lib.native().attention_nvfp4kv(q, k_blocks, v_blocks, block_tokens, k_cur, v_cur, heads, scale, out, key_splits, out_amax,
-                                           e2m1_max, e4m3_max, workspace)
+    return _lib.native().attention_nvfp4kv(q, _seq(k_blocks), _seq(v_blocks), int(block_tokens), k_cur, v_cur, heads, scale, out,
+                                           _opt_int(key_splits), out_amax, e2m1_max, e4m3_max, workspace)
 
 
 def dequantize_nvfp4(codes, sf, amax, rows, cols, cols_padded, dtype, e2m1_max, e4m3_max, rounding=DEQ_PYTORCH):
@@ -298,7 +307,9 @@ def dequantize_nvfp4(codes, sf, amax, rows, cols, cols_padded, dtype, e2m1_max, 
 
 def kv_dequant(values, scale_factors, amax, num_heads, block_token_size, dtype, e2m1_max, e4m3_max,
                rounding=DEQ_FUSED, out=None):
-    return _lib.native().kv_dequant(values, scale_factors, amax, num_heads, block_token_size, dtype, e2m1_max, e4m3_max, rounding, out)
+    if not isinstance(dtype, torch.dtype):
+        raise ValueError(f"Unsupported fused KV dequant dtype: {dtype}")
+    return _lib.native().kv_dequant(_seq(values), _seq(scale_factors), _seq(amax), num_heads, block_token_size, dtype, e2m1_max, e4m3_max, rounding, out)
 
 
 def gemm_nvfp4(a_codes, a_sf, a_amax, a_rule, b_codes, b_sf, b_amax, b_rule, m, n, k, *, out=None, alpha=None,
@@ -310,8 +321,9 @@ def gemm_nvfp4(a_codes, a_sf, a_amax, a_rule, b_codes, b_sf, b_amax, b_rule, m, 
     under the tensor amax ``requant_amax`` (fp32 [1], known before the call); with ``store_out=False`` the bf16
     result itself is not written and None is returned."""
     q_codes, q_sf = requant if requant is not None else (None, None)
-    return _lib.native().gemm(a_codes, a_sf, a_amax, a_rule, b_codes, b_sf, b_amax, b_rule, m, n, k, out, alpha, bias, act, residual, gate,
-                              frame_rows, out_amax, row_offset, tile, q_codes, q_sf, requant_amax, store_out)
+    frame_rows, row_offset = (int(frame_rows), int(row_offset)) if gate is not None else (0, 0)        # read with a gate only
+    return _lib.native().gemm(a_codes, a_sf, a_amax, a_rule, b_codes, b_sf, b_amax, b_rule, m, n, k, out, alpha, bias, int(act), residual, gate,
+                              frame_rows, out_amax, row_offset, int(tile), q_codes, q_sf, requant_amax if requant is not None else None, store_out)
 
 
 def gemm_nvfp4_grouped(a_codes, a_sf, a_amax, a_rule, b_codes, b_sf, b_amax, b_rule, m, n_each, k, outs, *, bias=None, act=0,
@@ -320,5 +332,5 @@ def gemm_nvfp4_grouped(a_codes, a_sf, a_amax, a_rule, b_codes, b_sf, b_amax, b_r
     ``b_sf`` are the weights concatenated along N, ``b_amax`` an fp32 tensor with one amax per weight,
     ``outs`` the output tensors (bf16 [m, n_each], any row stride), ``out_amax`` a list of fp32 [1]
     tensors or None per output."""
-    _lib.native().gemm_grouped(a_codes, a_sf, a_amax, a_rule, b_codes, b_sf, b_amax, b_rule, m, n_each, k, outs, bias, act, out_amax)
+    _lib.native().gemm_grouped(a_codes, a_sf, a_amax, a_rule, b_codes, b_sf, b_amax, b_rule, m, n_each, k, _seq(outs), bias, int(act), _seq(out_amax))
     return outs

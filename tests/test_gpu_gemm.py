@@ -415,3 +415,14 @@ def test_fp16_linear_with_bias():
     got = m(x)
     no_bias = L.fp4_matmul(L.quantize_to_fp4(x), m[0].quantized_weight())
     assert torch.equal(got, no_bias + bias.bfloat16())
+
+
+def test_linear_activation_rule_assigned_by_name():
+    m = torch.nn.Sequential(torch.nn.Linear(512, 256, device="cuda", dtype=torch.bfloat16))
+    L.quantize_model_with_filter(m, materialize_for_inference=True, verbose=False)
+    x = util.config_activation(20, 512, seed=4).cuda()
+    outs = []
+    for rule in (L.ScaleRule.mae, "mae"):
+        m[0].config.activation_scale_rule = rule
+        outs.append(m(x))
+    assert torch.equal(*outs)

@@ -115,3 +115,30 @@ def test_kernels_read_global_memory_with_ordinary_loads():
     for name in sorted(os.listdir(src)):
         code = re.sub(r"//.*", "", open(os.path.join(src, name)).read())
         assert not re.search(r"__ldg\s*\(|ld\.global\.nc|const\s+[\w:]+\s*\*\s*__restrict__", code), name
+
+
+def test_operations_take_the_argument_forms_they_took():
+    """Integers given as floats, blocks as dictionary values or a stacked tensor, unused arguments of any kind: such calls get as far as the
+    device check (CPU tensors here)."""
+    from longlive_b200 import ops
+    u8, f32, bf = torch.zeros(128, 128, dtype=torch.uint8), torch.zeros(1), torch.zeros(128, 256, dtype=torch.bfloat16)
+    blocks = {"a": L.QuantizedTensor(torch.zeros(128, 64, dtype=torch.uint8), torch.zeros(1024, dtype=torch.uint8), f32, "nvfp4", (128, 128), "mse")}
+    kv, sc, am = torch.zeros(2, 128, 64, dtype=torch.uint8), torch.zeros(2, 1024, dtype=torch.uint8), torch.zeros(2)
+    gemm = (u8, u8, f32, 3, u8, u8, f32, 3, 128, 128, 256)
+    calls = [
+        lambda: ops.gemm_nvfp4(*gemm, act=1.0, tile=128.0, residual=bf, gate=bf, frame_rows=880.0, row_offset=2.0),
+        lambda: ops.gemm_nvfp4(*gemm, frame_rows=None, row_offset=None, requant_amax="unused"),
+        lambda: ops.gemm_nvfp4_grouped(*gemm, {"q": bf, "k": bf}.values(), act=0.0, out_amax={"q": None, "k": f32}.values()),
+        lambda: ops.adaln_quantize_nvfp4(bf, bf, bf, 64.0, 3, row_offset=0.0, phase=0.0),
+        lambda: ops.layernorm_quantize_nvfp4(bf, bf[0], bf[0], 3, phase=0.0),
+        lambda: ops.attention_bf16(bf, bf, bf, 2, key_splits=1.0),
+        lambda: ops.attention_nvfp4kv(bf, blocks.values(), blocks.values(), 128.0, bf, bf, 2, key_splits=1.0),
+        lambda: ops.kv_dequant(kv, sc, am, 1, 128, torch.bfloat16, 6, 256),
+        lambda: ops.quantize_nvfp4(bf, 3, f32, amax_given=1),
+    ]
+    for i, call in enumerate(calls):
+        with pytest.raises(ValueError, match="CUDA tensor"):
+            call()
+            pytest.fail(f"call {i}")
+    with pytest.raises(ValueError):
+        ops.kv_dequant(kv, sc, am, 1, 128, "bfloat16", 6, 256)
