@@ -120,6 +120,10 @@ def native():
         except ImportError as exc:
             raise LibraryMissing("longlive_b200/_native.so is missing or was built for another PyTorch: build it with "
                                  f"`python -m longlive_b200.build` ({exc})") from exc
+        import torch
+        if mod.torch_version != torch.__version__:
+            raise LibraryMissing(f"longlive_b200/_native.so was built for PyTorch {mod.torch_version}, this is {torch.__version__}: "
+                                 "build it with `python -m longlive_b200.build`")
         _native = mod
     return _native
 

@@ -3,8 +3,8 @@
 
 ``python -m longlive_b200.build`` compiles every ``csrc/*.cu`` into one object each (in
 parallel) and links them into ``longlive_b200/libllnvfp4.so``, then ``csrc/binding.cpp`` into
-``longlive_b200/_native.so``.  Objects are rebuilt only when a source or header is newer.  nvcc
-cross-compiles without a GPU.
+``longlive_b200/_native.so``.  Objects are rebuilt only when a source or header is newer, the binding
+also when PyTorch, Python or its compile command is another.  nvcc cross-compiles without a GPU.
 """
 from __future__ import annotations
 
@@ -20,6 +20,7 @@ CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(PKG, "build")
 LIB = os.path.join(PKG, "libllnvfp4.so")
 NATIVE = os.path.join(PKG, "_native.so")
+NATIVE_STAMP = os.path.join(OBJ, "_native.stamp")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -39,24 +40,32 @@ def _newest(paths) -> float:
 
 
 def _build_binding(verbose: bool, force: bool) -> None:
-    src = os.path.join(CSRC, "binding.cpp")
-    newest = _newest([src, os.path.join(PKG, "..", "include", "llnvfp4.h")])
-    if not force and os.path.exists(NATIVE) and os.path.getmtime(NATIVE) >= newest:
-        return
     import sysconfig
     import torch
     from torch.utils.cpp_extension import include_paths, library_paths
+    src = os.path.join(CSRC, "binding.cpp")
     cuda_home = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
     inc = [*include_paths(), os.path.join(cuda_home, "include"), sysconfig.get_paths()["include"]]
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_native",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-isystem{p}" for p in inc), src, "-o", NATIVE,
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DLLNV_TORCH_VERSION="{torch.__version__}"',
+           *(f"-isystem{p}" for p in inc), src, "-o", NATIVE,
            f"-L{PKG}", "-lllnvfp4", "-Wl,-rpath,$ORIGIN", *(f"-L{p}" for p in library_paths()), "-lc10", "-lc10_cuda", "-ltorch_cpu",
            "-ltorch", "-ltorch_python"]
+    # what the binary was built for and how: it is tied to one PyTorch and one Python, which no source time shows
+    stamp = "\n".join([torch.__version__, sysconfig.get_config_var("SOABI") or "", *(a.replace(PKG, "<pkg>") for a in cmd)])
+    newest = _newest([src, os.path.join(PKG, "..", "include", "llnvfp4.h")])
+    if not force and os.path.exists(NATIVE) and os.path.getmtime(NATIVE) >= newest and os.path.exists(NATIVE_STAMP):
+        with open(NATIVE_STAMP) as f:
+            if f.read() == stamp:
+                return
     r = subprocess.run(cmd, capture_output=True, text=True)
     if verbose or r.returncode != 0:
         sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
     if r.returncode != 0:
         raise RuntimeError("build of _native.so failed")
+    os.makedirs(OBJ, exist_ok=True)
+    with open(NATIVE_STAMP, "w") as f:
+        f.write(stamp)
 
 
 def build(verbose: bool = False, force: bool = False) -> str:

@@ -505,6 +505,7 @@ uintptr_t current_stream(int device) { return reinterpret_cast<uintptr_t>(c10::c
 
 PYBIND11_MODULE(_native, m) {
   using Unlocked = py::call_guard<py::gil_scoped_release>;
+  m.attr("torch_version") = LLNV_TORCH_VERSION;
   m.def("quantize", &quantize, Unlocked());
   m.def("quantize_pair", &quantize_pair, Unlocked());
   m.def("adaln_quantize", &adaln_quantize, Unlocked());

@@ -142,3 +142,29 @@ def test_operations_take_the_argument_forms_they_took():
             pytest.fail(f"call {i}")
     with pytest.raises(ValueError):
         ops.kv_dequant(kv, sc, am, 1, 128, "bfloat16", 6, 256)
+
+
+def test_binding_is_rebuilt_for_another_pytorch(libpath, monkeypatch, tmp_path):
+    """The binary is tied to one PyTorch and Python: the build looks at them and not at source times alone, and a binary of another one
+    is not used."""
+    commands = []
+
+    class Done:
+        returncode, stdout, stderr = 0, "", ""
+
+    monkeypatch.setattr(build.subprocess, "run", lambda cmd, **kw: commands.append(cmd) or Done)
+    build._build_binding(False, False)
+    assert not commands                                   # as it was just built
+    monkeypatch.setattr(build, "NATIVE_STAMP", str(tmp_path / "stamp"))
+    build._build_binding(False, False)
+    assert len(commands) == 1                             # no record of what it was built for
+    build._build_binding(False, False)
+    assert len(commands) == 1
+    with monkeypatch.context() as m:
+        m.setattr(torch, "__version__", "0.0.0")
+        build._build_binding(False, False)
+        assert len(commands) == 2
+        m.setattr(_lib, "_native", None)
+        with pytest.raises(_lib.LibraryMissing, match="0.0.0"):
+            _lib.native()
+    assert _lib.native().torch_version == torch.__version__
