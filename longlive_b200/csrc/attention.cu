@@ -545,62 +545,62 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   }
 }
 
-// Merges the key splits: out = sum_z 2^((m_z - M) c) O_z / sum_z 2^((m_z - M) c) l_z with M = max_z m_z.
-// A warp merges kCombineRows consecutive query rows of one (query tile, head) item, a lane owns four of the 128 channels; the
-// rows' loads are independent, so that several are in flight.  Only items that were cut are visited (first_item: the first one;
-// 0 with uniform splits).  L2 / launch bound: 9 us for the 116 cut items of the shape above (18 us with one row per warp and a
-// warp for every row of the output).
-constexpr int kCombineRows = 4;
-__global__ void __launch_bounds__(256) attention_combine_kernel(const float* part_o, const float* part_ml,
-                                                                int nsplit, int64_t Lq, int heads, float scale_log2,
-                                                                uint16_t* __restrict__ out, int64_t ldo, float* __restrict__ out_amax,
-                                                                int first_item, int q_tiles) {
+// Merges the key splits: out = sum_z 2^((m_z - M) c) O_z / sum_z 2^((m_z - M) c) l_z with M = max_z m_z, z in order.
+// One warp per query row of a (query tile, head) item, a lane owns four of the 128 channels.  Only items that were cut are visited
+// (first_item: the first one; 0 with uniform splits).  Bound by latency: lane z holds (m_z, l_z), so that the weights cost one round of
+// loads whatever the number of splits, and the outputs of four splits are loaded at a time.  us, cold caches, 1980 rows in 6 parts / 16896 in
+// 2 / 29696 in 2: 4.6 / 7.4 / 10.9; four rows a warp with the loads of one split at a time 17.4 / 9.9 / 14, two rows 5.2 / 7.5 / 10.5.
+__global__ void __launch_bounds__(256) attention_combine_kernel(const float* part_o, const float* part_ml, int nsplit, int64_t Lq, int heads,
+                                                                float scale_log2, uint16_t* __restrict__ out, int64_t ldo,
+                                                                float* __restrict__ out_amax, int first_item, int q_tiles) {
   pdl_begin();
+  constexpr int kBatch = 4;
   const int lane = threadIdx.x & 31;
-  const int item = first_item + (int)blockIdx.x / (kBQ / (8 * kCombineRows));
+  const int item = first_item + (int)blockIdx.x / (kBQ / 8);
   const int head = item / q_tiles;
-  const int64_t row0 = (int64_t)(item % q_tiles) * kBQ + ((int)blockIdx.x % (kBQ / (8 * kCombineRows))) * (8 * kCombineRows) +
-                       (threadIdx.x >> 5) * kCombineRows;
-  const int64_t stride = Lq * heads;
-  float mmax[kCombineRows], lsum[kCombineRows];
-  float4 acc[kCombineRows];
+  const int64_t row = (int64_t)(item % q_tiles) * kBQ + ((int)blockIdx.x % (kBQ / 8)) * 8 + (threadIdx.x >> 5);
+  if (row >= Lq) return;                                        // the whole warp
+  const int64_t unit = row * heads + head, stride = Lq * heads;
+  float2 ml[2];                                                 // of splits lane and lane + 32 (at most 64)
 #pragma unroll
-  for (int r = 0; r < kCombineRows; ++r) {
-    mmax[r] = -INFINITY;
-    lsum[r] = 0.f;
-    acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int h = 0; h < 2; ++h) {
+    ml[h] = make_float2(-INFINITY, 0.f);
+    if (lane + 32 * h < nsplit) ml[h] = ld_global(reinterpret_cast<const float2*>(part_ml + ((lane + 32 * h) * stride + unit) * 2));
   }
-  for (int z = 0; z < nsplit; ++z)
+  float4 o[kBatch];
+  auto load = [&](int z0) {
 #pragma unroll
-    for (int r = 0; r < kCombineRows; ++r)
-      if (row0 + r < Lq) mmax[r] = fmaxf(mmax[r], ld_global(part_ml + (z * stride + (row0 + r) * heads + head) * 2));
-#pragma unroll 2
-  for (int z = 0; z < nsplit; ++z)
+    for (int i = 0; i < kBatch; ++i)
+      if (z0 + i < nsplit) o[i] = ld_global(reinterpret_cast<const float4*>(part_o + ((z0 + i) * stride + unit) * kD) + lane);
+  };
+  load(0);
+  const float mmax = warp_max(fmaxf(ml[0].x, ml[1].x));
 #pragma unroll
-    for (int r = 0; r < kCombineRows; ++r) {
-      if (row0 + r >= Lq) continue;
-      const int64_t unit = z * stride + (row0 + r) * heads + head;
-      const float2 ml = ld_global(reinterpret_cast<const float2*>(part_ml + unit * 2));
-      const float w = exp2f((ml.x - mmax[r]) * scale_log2);
-      const float4 o = ld_global(reinterpret_cast<const float4*>(part_o + unit * kD) + lane);
-      acc[r].x = __fmaf_rn(w, o.x, acc[r].x);
-      acc[r].y = __fmaf_rn(w, o.y, acc[r].y);
-      acc[r].z = __fmaf_rn(w, o.z, acc[r].z);
-      acc[r].w = __fmaf_rn(w, o.w, acc[r].w);
-      lsum[r] = __fmaf_rn(w, ml.y, lsum[r]);
+  for (int h = 0; h < 2; ++h) ml[h].x = exp2f((ml[h].x - mmax) * scale_log2);       // the split's weight
+  float lsum = 0.f;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int z0 = 0; z0 < nsplit; z0 += kBatch) {
+    if (z0 > 0) load(z0);
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      const int z = z0 + i;
+      if (z >= nsplit) break;
+      const float w = __shfl_sync(0xFFFFFFFFu, z < 32 ? ml[0].x : ml[1].x, z & 31);
+      const float l = __shfl_sync(0xFFFFFFFFu, z < 32 ? ml[0].y : ml[1].y, z & 31);
+      acc.x = __fmaf_rn(w, o[i].x, acc.x);
+      acc.y = __fmaf_rn(w, o[i].y, acc.y);
+      acc.z = __fmaf_rn(w, o[i].z, acc.z);
+      acc.w = __fmaf_rn(w, o[i].w, acc.w);
+      lsum = __fmaf_rn(w, l, lsum);
     }
-  uint32_t m2 = 0u;
-#pragma unroll
-  for (int r = 0; r < kCombineRows; ++r) {
-    if (row0 + r >= Lq) continue;
-    const float inv = 1.f / lsum[r];
-    uint2 packed;
-    packed.x = pack2(acc[r].x * inv, acc[r].y * inv);
-    packed.y = pack2(acc[r].z * inv, acc[r].w * inv);
-    *reinterpret_cast<uint2*>(out + (row0 + r) * ldo + (int64_t)head * kD + lane * 4) = packed;
-    m2 = __vmaxu2(m2, __vmaxu2(packed.x & 0x7FFF7FFFu, packed.y & 0x7FFF7FFFu));
   }
+  const float inv = 1.f / lsum;
+  uint2 packed;
+  packed.x = pack2(acc.x * inv, acc.y * inv);
+  packed.y = pack2(acc.z * inv, acc.w * inv);
+  *reinterpret_cast<uint2*>(out + row * ldo + (int64_t)head * kD + lane * 4) = packed;
   if (out_amax) {
+    const uint32_t m2 = __vmaxu2(packed.x & 0x7FFF7FFFu, packed.y & 0x7FFF7FFFu);
     const float a = warp_max(__uint_as_float(max(m2 & 0xFFFFu, m2 >> 16) << 16));
     if (lane == 0 && a > 0.f) atomic_max_nonneg(out_amax, a);
   }
@@ -766,7 +766,7 @@ int attention_launch(const void* q, int64_t Lq, int64_t ldq, const void* k, cons
   if (rc == LLNV_OK) rc = launch_tiles(grid, stream, tmQ, tmK, tmV, tmK2, tmV2, tmO, p);
   if (rc == LLNV_OK && zdim > 1) {
     const int first_item = tail_cut > 0 ? p.tail_first : 0;
-    const int64_t blocks = ((int64_t)q_tiles * heads - first_item) * (kBQ / (8 * kCombineRows));
+    const int64_t blocks = ((int64_t)q_tiles * heads - first_item) * (kBQ / 8);
     launch_k(attention_combine_kernel, (unsigned)blocks, 256, 0, stream, p.part_o, p.part_ml, zdim, Lq, heads, p.scale_log2, (uint16_t*)out, ldo,
              out_amax, first_item, q_tiles);
     rc = launch_status("attention_combine_kernel");

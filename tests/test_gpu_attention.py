@@ -399,3 +399,17 @@ def test_attention_non_finite_query_stays_in_its_row():
     want = torch.zeros(lq, heads * 128, dtype=torch.bool, device="cuda")
     want[170, :128] = True
     assert torch.equal(out.isnan(), want)
+
+
+@pytest.mark.parametrize("splits", [2, 3, 4, 5, 9, 33, 64])
+def test_merge_of_many_splits(splits):
+    """Every count that ends a batch of four or a warp's 32 lanes: the merge of the parts agrees with the unsplit call to fp32 rounding of the
+    sums, seen behind the bf16 rounding of P and of the output (a bf16 ulp where it moves one, 2^-8 of the value)."""
+    heads, lq, lk = 2, 300, 64 * 128 + 5
+    g = torch.Generator(device="cuda").manual_seed(splits)
+    q, k, v = (torch.randn(n, heads * 128, generator=g, device="cuda").bfloat16() for n in (lq, lk, lk))
+    amax = [torch.zeros(1, device="cuda") for _ in range(2)]
+    ref = ops.attention_bf16(q, k, v, heads, key_splits=1, out_amax=amax[0]).float()
+    out = ops.attention_bf16(q, k, v, heads, key_splits=splits, out_amax=amax[1]).float()
+    assert float((out - ref).norm() / ref.norm()) < 4e-3
+    assert float(amax[1]) == float(out.abs().max()) and float(amax[0]) == float(ref.abs().max())
