@@ -303,7 +303,8 @@ int llnv_attention_key_splits(int64_t Lq, int64_t Lk, int heads);
  * sites wan_5b/modules/causal_model.py:557-600, 628-652), window assembly with torch.cat (:673-724) and
  * attention() (:781, wan_5b/modules/attention.py:241-254).  Here one launch expands the cached keys and
  * values of all blocks into the workspace, with the rounding of the fused dequantize kernel (LLNV_DEQ_FUSED),
- * and the attention kernel reads them there and the current chunk in place; the result equals llnv_kv_dequant
+ * and the attention kernel reads them there and the current chunk in place (where the workspace has no room for them,
+ * the attention kernel decodes the blocks as it loads them); the result equals llnv_kv_dequant
  * followed by llnv_attention_bf16_ex on the concatenated window bit for bit.
  *   k_codes / k_sf / k_amax / v_*: HOST arrays of num_blocks (<= 16) DEVICE pointers, passed to the kernel
  *   as launch parameters.  Codes must be 16-byte aligned, block_token_size >= 128.  num_blocks == 0 is llnv_attention_bf16_ex on
@@ -317,7 +318,8 @@ int llnv_attention_nvfp4kv(const void* q, int64_t Lq, int64_t ldq, const void* c
                            int64_t workspace_bytes, float* out_amax, llnv_stream_t stream);
 int64_t llnv_attention_workspace_bytes(int64_t Lq, int heads, int key_splits);
 /* Workspace of an llnv_attention_nvfp4kv call: the partial results of a split call plus the cached blocks expanded to bf16.
- * With less (down to llnv_attention_workspace_bytes) the call takes the expanded window from the stream-ordered allocator. */
+ * With less (down to llnv_attention_workspace_bytes, none for an unsplit call) the cached blocks are decoded inside the attention
+ * kernel instead: the same result bit for bit, slower on long windows, and nothing is allocated either way. */
 int64_t llnv_attention_nvfp4kv_workspace_bytes(int64_t Lq, int heads, int key_splits, int num_blocks, int block_token_size);
 
 /* Fused epilogue of the W4A4 GEMM.  All pointers are device pointers and optional (NULL = skip).

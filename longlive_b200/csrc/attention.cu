@@ -36,9 +36,22 @@
 //
 // The window may come in two pieces (keys [0, 128 * first_tiles) and the rest): the NVFP4 window of llnv_attention_nvfp4kv is
 // expanded to bf16 in a workspace by one dequantize launch (26 us of HBM time on the shape above) and read from there, while
-// the current chunk is read in place.  Decoding the cache inside this kernel's load stage instead repeats the decode for each
-// of a head's query tiles and is bound by shared-memory bandwidth (MMA operands plus the expanded tiles): it took 474 us with
-// four decode warps and 459 us with eight; where one query tile covers the chunk it saved 2 us of 36.
+// the current chunk is read in place.
+//
+// A call whose workspace has no room for the expanded window takes attention_kernel<true>, which needs none: four more warps
+// (12-15) decode the cached keys and values inside the load stage.  That repeats the decode for each of a head's query tiles and is
+// bound by shared-memory bandwidth (MMA operands plus the expanded tiles).  us with the expansion / without, 4 cached blocks and the
+// chunk: 2640 x 24 heads 371 / 467, 2640 x 12 190 / 250, 660 x 24 48 / 54, 660 x 3 25.5 / 27.4; 2 blocks, 2640 x 6 74.5 / 100.
+// Warp 0 loads Q and the K side, warp 3 the V side: the 128 x 64-byte code tile of the stage's next key tile (one box per cache block
+// the tile touches, at most two) goes into the tail of the K / V stage itself, which is free at that point.  Decode thread i owns key row i: it
+// takes the row's 64 code bytes from there and its 8 scale bytes from global memory (one tile ahead) and writes the bf16 row over the
+// stage in the swizzled layout the MMAs read, the bytes a TMA load of the expanded window would have put there.  The value of a code,
+//     bf16((e2m1 * e4m3) * (amax * fp32(1 / (e2m1_max * e4m3_max)))),
+// depends within one block only on scale byte and code: when a tile first touches a block, the eight bf16 magnitudes of each of the
+// 128 scale bytes go into a 2 KiB table (byte-split for prmt), and a row is decoded with byte permutes alone.  A tile that holds the last
+// cached keys and the first keys of the current chunk is built by these warps too; tiles in the current chunk come from TMA.  One
+// thread issues the MMAs of both halves, and the softmax reads its scores twice in a rolled loop: with the decode's code the
+// unrolled one overflows the instruction cache (467 -> 498 us).  Registers: load / MMA warpgroup 56, decode 104, softmax 176.
 //
 // Work split.  blockIdx.z = key split: with nsplit > 1 every (query tile, head) item is cut into nsplit equal ranges of key
 // tiles, each CTA writes unnormalised fp32 partials and (m, l), and attention_combine_kernel merges them (head shards with
@@ -74,10 +87,18 @@ constexpr uint32_t kVOff = kKOff + kStages * kTileBytes;
 constexpr uint32_t kBarOff = kVOff + kStages * kTileBytes;
 constexpr uint32_t kTmemCols = 512;
 constexpr int kMaxKvBlocks = 16;
+// attention_kernel<true>: decode tables behind the barriers, kTabSlots cache blocks x (K, V) x 128 scale bytes x 16 bytes
+constexpr int kTabSlots = 2;                      // a tile of 128 keys touches at most two cache blocks (blocks hold >= 128 tokens)
+constexpr uint32_t kCodeBytes = 128 * 64;         // code tile of one cache block: 128 key rows x 64 bytes, 64-byte swizzle
+constexpr uint32_t kCodeOff = kTileBytes - 2 * kCodeBytes;      // two code tiles in the tail of the stage they expand into
+constexpr uint32_t kTabOff = kBarOff + 1024;
+constexpr uint32_t kSmemBytesFused = kTabOff + kTabSlots * 2 * 128 * 16;
+static_assert(kSmemBytesFused <= 232448, "more shared memory than one CTA may use");
 
 constexpr uint32_t kSmemBytes = kBarOff + 1024;
 constexpr uint32_t kSCol = 0, kPCol = 128, kOCol = 256;      // one S tile, P_h at kPCol + 64 h, O_h at kOCol + 128 h
 constexpr int kThreads = 384;      // three warpgroups: load + MMA, softmax a, softmax b
+constexpr int kThreadsFused = 512; // and a fourth: decode
 
 struct AttnParams {
   int64_t Lq, Lk;
@@ -96,6 +117,33 @@ struct AttnParams {
   // key tiles [0, first_tiles) come from the first K / V tensors (rows from 0), the others from the second ones,
   // whose row second_row holds the first key of tile first_tiles
   int first_tiles, second_row;
+};
+
+// Tensor-memory columns of a half's scores and probabilities.  FUSED: a score buffer for each half, which the probabilities overwrite
+// (S(j + 1) is issued behind the products of tile j).  The K tiles are late there, and with the shared buffer one that half a has read
+// waits for half b's turn: 2640 x 7920 x 6 heads 111 us, with a buffer each 99.
+template <bool FUSED>
+__device__ __forceinline__ uint32_t s_col(int h) { return kSCol + (FUSED ? 128 * h : 0); }
+template <bool FUSED>
+__device__ __forceinline__ uint32_t p_col(int h) { return FUSED ? kSCol + 128 * h : kPCol + 64 * h; }
+
+// The cached blocks of an attention_kernel<true> launch (oldest first); the kernel without them takes an empty table.
+template <bool FUSED>
+struct KvTable {};
+template <>
+struct KvTable<true> {
+  const uint8_t* k_sf[kMaxKvBlocks];
+  const float* k_amax[kMaxKvBlocks];
+  const uint8_t* v_sf[kMaxKvBlocks];
+  const float* v_amax[kMaxKvBlocks];
+  // codes of block b viewed as [block_tokens, heads * 64 bytes]: box = 128 tokens x the 64 bytes of one head
+  CUtensorMap k_codes[kMaxKvBlocks];
+  CUtensorMap v_codes[kMaxKvBlocks];
+  int n_cached, block_tokens;
+  float inv_denom;             // fp32(1 / (e2m1_max * e4m3_max))
+  const uint16_t* k_cur;       // current chunk: rows of the tile it shares with the cache
+  const uint16_t* v_cur;
+  int64_t ldk, ldv;
 };
 
 // The CTA's share of the key tiles: [j0, j0 + nt).  False: this CTA has nothing to do (tail balancing, whole item).
@@ -120,6 +168,81 @@ template <int N>
 __device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N>
 __device__ __forceinline__ void setmaxnreg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// What a decode thread keeps of its key row between the prefetch and the decode.
+struct RowInfo {
+  uint32_t ksf[2], vsf[2];      // kind 0: the row's 8 K and 8 V scale bytes
+  int kind;                     // 0 = cache block, 1 = current chunk, 2 = beyond the window
+  int where;                    // kind 0: row inside the staged code tiles (128.. = second tile) | table slot << 8;
+                                // kind 1: row of the current chunk
+};
+
+// Decode table of one (cache block, scale byte): the bf16 magnitudes of the eight E2M1 magnitudes
+// {0, .5, 1, 1.5, 2, 3, 4, 6} under that scale, computed as decode16<LLNV_DEQ_FUSED> of the standalone
+// dequantize kernel computes them, stored byte-split: x = low bytes of magnitudes 0..3, y = low bytes of
+// 4..7, z / w = the high bytes.
+__device__ __forceinline__ uint4 decode_table_entry(uint32_t scale_byte, float g) {
+  const float s = e4m3_to_float(scale_byte);
+  const float mags[8] = {0.f, 0.5f, 1.f, 1.5f, 2.f, 3.f, 4.f, 6.f};
+  uint32_t pk[4];
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+    pk[m] = pack_bf16x2(__fmul_rn(__fmul_rn(mags[2 * m], s), g), __fmul_rn(__fmul_rn(mags[2 * m + 1], s), g));
+  uint4 t;
+  t.x = __byte_perm(pk[0], pk[1], 0x6420);
+  t.y = __byte_perm(pk[2], pk[3], 0x6420);
+  t.z = __byte_perm(pk[0], pk[1], 0x7531);
+  t.w = __byte_perm(pk[2], pk[3], 0x7531);
+  return t;
+}
+
+// 8 codes (one word) -> 8 bf16 (16 bytes) with the table entry `t` of the codes' scale byte: four byte lookups
+// (low / high bytes of codes 0..3 and 4..7), the sign bits, four interleaves.
+__device__ __forceinline__ uint4 decode_word(uint32_t w, const uint4& t) {
+  const uint32_t sel = w & 0x77777777u;             // magnitude indices of codes 0..3 (low half) and 4..7
+  const uint32_t selb = sel >> 16;
+  const uint32_t w4 = w << 4;                       // bit 7 of byte k: sign of code 2k (of w: sign of code 2k+1)
+  const uint32_t lo_a = __byte_perm(t.x, t.y, sel), lo_b = __byte_perm(t.x, t.y, selb);
+  uint32_t hi_a = __byte_perm(t.z, t.w, sel), hi_b = __byte_perm(t.z, t.w, selb);
+  hi_a |= __byte_perm(w4, w, 0x5140) & 0x80808080u;
+  hi_b |= __byte_perm(w4, w, 0x7362) & 0x80808080u;
+  return make_uint4(__byte_perm(lo_a, hi_a, 0x5140), __byte_perm(lo_a, hi_a, 0x7362), __byte_perm(lo_b, hi_b, 0x5140),
+                    __byte_perm(lo_b, hi_b, 0x7362));
+}
+
+// Decode a cached row (code words w[0..15], scale bytes sf0 | sf1) into row i of a K / V stage: two halves of 64
+// channels, rows of 128 bytes, 16-byte chunks XOR-swizzled with the row index as a TMA load with the 128-byte
+// swizzle writes them.  `tab` is the row's block's table (128 entries of 16 bytes) in shared memory.  The loop
+// over the four 32-channel groups stays rolled (the words rotate through w[0..3]): unrolled, this code and the
+// softmax's together overflow the instruction cache.
+__device__ __forceinline__ void decode_row(uint32_t (&w)[16], uint32_t sf0, uint32_t sf1, const uint8_t* tab, uint8_t* stage, int i) {
+  uint8_t* dst = stage + i * 128;
+  const int x = i & 7;
+#pragma unroll 1
+  for (int c = 0; c < 4; ++c) {                       // 32 channels: two scale bytes, four 16-byte chunks
+    const uint32_t sfw = (c & 2 ? sf1 : sf0) >> (16 * (c & 1));
+    // table entries of the two scale bytes (bit 7 of a UE4M3 scale is never set): byte * 16
+    const uint4 t0 = *reinterpret_cast<const uint4*>(tab + ((sfw << 4) & 0x7F0u));
+    const uint4 t1 = *reinterpret_cast<const uint4*>(tab + ((sfw >> 4) & 0x7F0u));
+    uint8_t* half = dst + (c >> 1) * kHalfBytes;
+    const int k0 = (c & 1) * 4;                       // first chunk of the group inside its half
+    *reinterpret_cast<uint4*>(half + (((k0 + 0) ^ x) << 4)) = decode_word(w[0], t0);
+    *reinterpret_cast<uint4*>(half + (((k0 + 1) ^ x) << 4)) = decode_word(w[1], t0);
+    *reinterpret_cast<uint4*>(half + (((k0 + 2) ^ x) << 4)) = decode_word(w[2], t1);
+    *reinterpret_cast<uint4*>(half + (((k0 + 3) ^ x) << 4)) = decode_word(w[3], t1);
+#pragma unroll
+    for (int k = 0; k < 12; ++k) w[k] = w[k + 4];
+  }
+}
+
+// Row i of a stage from 128 bf16 values in global memory (src == nullptr: zeros).
+__device__ __forceinline__ void copy_row(const uint16_t* src, uint8_t* stage, int i) {
+#pragma unroll 4
+  for (int chunk = 0; chunk < 16; ++chunk) {
+    const uint4 v = src ? ld_global(reinterpret_cast<const uint4*>(src) + chunk) : make_uint4(0u, 0u, 0u, 0u);
+    *reinterpret_cast<uint4*>(stage + (chunk >> 3) * kHalfBytes + i * 128 + (((chunk & 7) ^ (i & 7)) << 4)) = v;
+  }
+}
 
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -186,13 +309,14 @@ __host__ __device__ constexpr bool poly_pair(int p) { return p % 4 == 1; }
 
 // Maximum of a row's scores: independent chains of three-input maxima.  NaN if a score is NaN, whatever its column: the FMA-pipe
 // exponential would lose it.
-__device__ __forceinline__ float row_max(const uint32_t (&sr)[4][32]) {
+template <int G>
+__device__ __forceinline__ float row_max(const uint32_t (&sr)[G][32]) {
   constexpr int kChains = 8;
   float mx[kChains];
 #pragma unroll
   for (int i = 0; i < kChains; ++i) mx[i] = fmax2(__uint_as_float(sr[0][2 * i]), __uint_as_float(sr[0][2 * i + 1]));
 #pragma unroll
-  for (int i = 2 * kChains; i < 128; i += 2) {
+  for (int i = 2 * kChains; i < 32 * G; i += 2) {
     float& x = mx[(i >> 1) % kChains];
     x = fmax3(x, __uint_as_float(sr[i >> 5][i & 31]), __uint_as_float(sr[i >> 5][(i & 31) + 1]));
   }
@@ -204,9 +328,10 @@ __device__ __forceinline__ float row_max(const uint32_t (&sr)[4][32]) {
 }
 
 // Columns at or beyond `valid` become -inf (only the last key tile of a window can be ragged).
-__device__ __forceinline__ void mask_scores(uint32_t (&sr)[4][32], int valid) {
+template <int G>
+__device__ __forceinline__ void mask_scores(uint32_t (&sr)[G][32], int valid) {
 #pragma unroll
-  for (int g = 0; g < 4; ++g) {
+  for (int g = 0; g < G; ++g) {
     const int nv = valid - 32 * g;                // valid columns of this group of 32
     const uint32_t keep = nv >= 32 ? 0xFFFFFFFFu : (nv <= 0 ? 0u : ((1u << nv) - 1u));
 #pragma unroll
@@ -309,10 +434,33 @@ __device__ __forceinline__ void write_output(const AttnParams& p, const CUtensor
   if (lane == 0) bulk_wait<0>();
 }
 
-__global__ void __launch_bounds__(kThreads, 1)
+// S = Q K^T of one half and key tile
+__device__ __forceinline__ void issue_scores(uint32_t s_tmem, uint32_t q_addr, uint32_t k_addr) {
+  constexpr uint32_t idesc = make_idesc_bf16(kHQ, kBK, 0, 0);     // A, B K-major
+#pragma unroll
+  for (int ks = 0; ks < 8; ++ks) {
+    // 16 channels per MMA: 32 bytes along the swizzled 128-byte row, second half after 4 steps
+    const uint32_t off = (ks >> 2) * kHalfBytes + (ks & 3) * 32;
+    mma_f16_ss(s_tmem, make_kmajor_sw128_desc(q_addr + off), make_kmajor_sw128_desc(k_addr + off), idesc, ks != 0);
+  }
+}
+// O (+)= P V of one half, keys 16 * KS0 .. 16 * KS1 - 1 of a tile
+template <int KS0, int KS1>
+__device__ __forceinline__ void issue_products(uint32_t o_tmem, uint32_t p_tmem, uint32_t v_addr, bool accumulate) {
+  constexpr uint32_t idesc = make_idesc_bf16(kHQ, kD, 0, 1);      // B (V) MN-major
+#pragma unroll
+  for (int ks = KS0; ks < KS1; ++ks) {
+    // 16 keys per MMA: P columns 8*ks..8*ks+7 (two bf16 per column), V rows 16*ks.. (2048 bytes apart)
+    // V is MN-major: 64 channels contiguous per key row, the second 64 channels one half-tile further
+    mma_f16_ts(o_tmem, p_tmem + 8 * ks, make_smem_desc(v_addr + ks * 2048, kHalfBytes, 1024, 2), idesc, accumulate || ks != 0);
+  }
+}
+
+template <bool FUSED>
+__global__ void __launch_bounds__(FUSED ? kThreadsFused : kThreads, 1)
 attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                  const __grid_constant__ CUtensorMap tmK2, const __grid_constant__ CUtensorMap tmV2, const __grid_constant__ CUtensorMap tmO,
-                 const AttnParams p) {
+                 const AttnParams p, const __grid_constant__ KvTable<FUSED> tab) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* q_full = reinterpret_cast<uint64_t*>(smem + kBarOff);
   uint64_t* k_full = q_full + 1;
@@ -323,7 +471,9 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint64_t* s_free = s_full + 2;               // [2 halves]: the half has its scores in registers
   uint64_t* p_ready = s_free + 2;              // [2 halves][2 key groups of 64]
   uint64_t* pv_done = p_ready + 4;             // [2 halves][2 key groups]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 4);
+  uint64_t* kc_full = pv_done + 4;             // [kStages] code tiles of a K / V stage have landed (FUSED)
+  uint64_t* vc_full = kc_full + kStages;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(vc_full + kStages);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -345,9 +495,11 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     mbar_init(q_full, 1);
     for (int i = 0; i < kStages; ++i) {
       mbar_init(&k_full[i], 1);
-      mbar_init(&k_empty[i], n_half);
+      mbar_init(&k_empty[i], FUSED ? 1 : n_half);
       mbar_init(&v_full[i], 1);
-      mbar_init(&v_empty[i], n_half);
+      mbar_init(&v_empty[i], FUSED ? 1 : n_half);
+      mbar_init(&kc_full[i], 1);
+      mbar_init(&vc_full[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&s_full[i], 1);
@@ -378,61 +530,118 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const uint32_t tmem_base = *tmem_slot;
   // The register file is re-divided at the top of every warpgroup's branch (all four warps of a warpgroup execute the same
   // instruction; an increase waits for the other warpgroups' releases): 12 warps x 32 x 168 registers at launch = 64512 >=
-  // 128 x (80 + 2 x 208).
-  if (warp < 4) setmaxnreg_dec<80>();
+  // 128 x (80 + 2 x 208); FUSED: 16 warps x 32 x 128 = 65536 = 128 x (56 + 2 x 176 + 104).
+  if (warp < 4) setmaxnreg_dec<FUSED ? 56 : 80>();
 
-  if (warp == 0) {
+  if (warp == 0 || (FUSED && warp == 3)) {
     // ------------------------------------------------------------------ TMA producer
+    // FUSED: warp 0 loads Q and feeds the K stages, warp 3 feeds the V stages, so that neither side queues behind the other's stage
+    const bool do_k = warp == 0, do_v = !FUSED || warp == 3;
     if (elect_one()) {
       const int col = head * kD;
-      mbar_arrive_expect_tx(q_full, n_half * kTileBytes);
-      for (int h = 0; h < n_half; ++h) {
-        tma_load_2d(smem + kQOff + h * kTileBytes, &tmQ, col, qt * kBQ + h * kHQ, q_full);
-        tma_load_2d(smem + kQOff + h * kTileBytes + kHalfBytes, &tmQ, col + 64, qt * kBQ + h * kHQ, q_full);
+      if (do_k) {
+        mbar_arrive_expect_tx(q_full, n_half * kTileBytes);
+        for (int h = 0; h < n_half; ++h) {
+          tma_load_2d(smem + kQOff + h * kTileBytes, &tmQ, col, qt * kBQ + h * kHQ, q_full);
+          tma_load_2d(smem + kQOff + h * kTileBytes + kHalfBytes, &tmQ, col + 64, qt * kBQ + h * kHQ, q_full);
+        }
+      }
+      // (block, token) of the first key of tile j, advanced tile by tile
+      int b0 = 0, tok0 = 0;
+      if constexpr (FUSED) {
+        b0 = (int)(((int64_t)j0 * kBK) / tab.block_tokens);
+        tok0 = (int)((int64_t)j0 * kBK - (int64_t)b0 * tab.block_tokens);
       }
       for (int j = 0; j < nt; ++j) {
         const int s = j % kStages;
         const uint32_t ph = (uint32_t)((j / kStages) & 1);
         const int t = j0 + j;
         const bool first = t < p.first_tiles;
+        if constexpr (FUSED) {
+          if (first) {
+            // a tile the decode warps build: its codes go into the tail of the (free) stage, one box of 128 token rows per cache
+            // block the tile touches; rows beyond a block's end arrive as zeros and are not used
+            const bool two = tok0 + kBK > tab.block_tokens && (int64_t)(b0 + 1) * tab.block_tokens < tab.n_cached;
+            const uint32_t bytes = two ? 2 * kCodeBytes : kCodeBytes;
+            uint8_t* stage = smem + (do_k ? kKOff : kVOff) + s * kTileBytes + kCodeOff;
+            uint64_t* full = do_k ? &kc_full[s] : &vc_full[s];
+            const CUtensorMap* codes = do_k ? tab.k_codes : tab.v_codes;
+            mbar_wait(do_k ? &k_empty[s] : &v_empty[s], ph ^ 1u, abort_flag, p.status, do_k ? 102u : 103u);
+            mbar_arrive_expect_tx(full, bytes);
+            tma_load_2d(stage, &codes[b0], head * 64, tok0, full);
+            if (two) tma_load_2d(stage + kCodeBytes, &codes[b0 + 1], head * 64, 0, full);
+            tok0 += kBK;
+            if (tok0 >= tab.block_tokens) { tok0 -= tab.block_tokens; ++b0; }
+            continue;
+          }
+        }
         const CUtensorMap* mk = first ? &tmK : &tmK2;
         const CUtensorMap* mv = first ? &tmV : &tmV2;
         const int krow = first ? t * kBK : (t - p.first_tiles) * kBK + p.second_row;
-        mbar_wait(&k_empty[s], ph ^ 1u, abort_flag, p.status, 100u);
-        mbar_arrive_expect_tx(&k_full[s], kTileBytes);
-        tma_load_2d(smem + kKOff + s * kTileBytes, mk, col, krow, &k_full[s]);
-        tma_load_2d(smem + kKOff + s * kTileBytes + kHalfBytes, mk, col + 64, krow, &k_full[s]);
-        mbar_wait(&v_empty[s], ph ^ 1u, abort_flag, p.status, 101u);
-        mbar_arrive_expect_tx(&v_full[s], kTileBytes);
-        tma_load_2d(smem + kVOff + s * kTileBytes, mv, col, krow, &v_full[s]);
-        tma_load_2d(smem + kVOff + s * kTileBytes + kHalfBytes, mv, col + 64, krow, &v_full[s]);
+        if (do_k) {
+          mbar_wait(&k_empty[s], ph ^ 1u, abort_flag, p.status, 100u);
+          mbar_arrive_expect_tx(&k_full[s], kTileBytes);
+          tma_load_2d(smem + kKOff + s * kTileBytes, mk, col, krow, &k_full[s]);
+          tma_load_2d(smem + kKOff + s * kTileBytes + kHalfBytes, mk, col + 64, krow, &k_full[s]);
+        }
+        if (do_v) {
+          mbar_wait(&v_empty[s], ph ^ 1u, abort_flag, p.status, 101u);
+          mbar_arrive_expect_tx(&v_full[s], kTileBytes);
+          tma_load_2d(smem + kVOff + s * kTileBytes, mv, col, krow, &v_full[s]);
+          tma_load_2d(smem + kVOff + s * kTileBytes + kHalfBytes, mv, col + 64, krow, &v_full[s]);
+        }
       }
     }
-  } else if (warp == 1 || warp == 2) {
+  } else if (FUSED && warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer of both halves
+    // A K tile is free as soon as both halves have read it, and one that is still being decoded holds up no products.
+    if (elect_one()) {
+      auto issue_qk = [&](int t, int h) {
+        const int s = t % kStages;
+        issue_scores(tmem_base + s_col<FUSED>(h), smem_u32(smem + kQOff + h * kTileBytes), smem_u32(smem + kKOff + s * kTileBytes));
+        tc_commit(&s_full[h]);
+        if (h == n_half - 1) tc_commit(&k_empty[s]);
+      };
+      mbar_wait(q_full, 0u, abort_flag, p.status, 201u);
+      mbar_wait(&k_full[0], 0u, abort_flag, p.status, 200u);
+      tc_fence_after();
+      for (int h = 0; h < n_half; ++h) issue_qk(0, h);
+      for (int j = 0; j < nt; ++j) {
+        const int s = j % kStages;
+        mbar_wait(&v_full[s], (uint32_t)((j / kStages) & 1), abort_flag, p.status, 203u);
+        for (int h = 0; h < n_half; ++h) {
+          mbar_wait(&p_ready[2 * h + 1], (uint32_t)(j & 1), abort_flag, p.status, 202u);
+          tc_fence_after();
+          issue_products<0, 8>(tmem_base + kOCol + 128 * h, tmem_base + p_col<FUSED>(h), smem_u32(smem + kVOff + s * kTileBytes), j != 0);
+          tc_commit(&pv_done[2 * h + 1]);
+          if (h == n_half - 1) tc_commit(&v_empty[s]);
+          if (j + 1 < nt) {
+            if (h == 0) {
+              mbar_wait(&k_full[(j + 1) % kStages], (uint32_t)(((j + 1) / kStages) & 1), abort_flag, p.status, 204u);
+              tc_fence_after();
+            }
+            issue_qk(j + 1, h);
+          }
+        }
+      }
+    }
+  } else if (!FUSED && (warp == 1 || warp == 2)) {
     // ------------------------------------------------------------------ MMA issuers, one per half
     const int h = warp - 1;
     if (h < n_half && elect_one()) {
-      constexpr uint32_t idesc_qk = make_idesc_bf16(kHQ, kBK, 0, 0);     // A, B K-major
-      constexpr uint32_t idesc_pv = make_idesc_bf16(kHQ, kD, 0, 1);      // B (V) MN-major
       const uint32_t q_addr = smem_u32(smem + kQOff + h * kTileBytes);
-      const uint32_t s_tmem = tmem_base + kSCol, p_tmem = tmem_base + kPCol + 64 * h, o_tmem = tmem_base + kOCol + 128 * h;
+      const uint32_t s_tmem = tmem_base + s_col<FUSED>(h), p_tmem = tmem_base + p_col<FUSED>(h), o_tmem = tmem_base + kOCol + 128 * h;
       const int before = n_half == 2 ? h ^ 1 : 0;          // whose scores occupy the S buffer before mine do
 
       // S of tile t: the buffer must have been read by its previous user (half b's tile t - 1 before half a's tile t, half
       // a's tile t before half b's)
       auto issue_qk = [&](int t) {
         const int s = t % kStages;
-        const uint32_t k_addr = smem_u32(smem + kKOff + s * kTileBytes);
         mbar_wait(&k_full[s], (uint32_t)((t / kStages) & 1), abort_flag, p.status, 204u);
         const int use = h == 1 ? t : t - 1;
         if (use >= 0) mbar_wait(&s_free[before], (uint32_t)(use & 1), abort_flag, p.status, 205u);
         tc_fence_after();
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          // 16 channels per MMA: 32 bytes along the swizzled 128-byte row, second half after 4 steps
-          const uint32_t off = (ks >> 2) * kHalfBytes + (ks & 3) * 32;
-          mma_f16_ss(s_tmem, make_kmajor_sw128_desc(q_addr + off), make_kmajor_sw128_desc(k_addr + off), idesc_qk, ks != 0);
-        }
+        issue_scores(s_tmem, q_addr, smem_u32(smem + kKOff + s * kTileBytes));
         tc_commit(&s_full[h]);
         tc_commit(&k_empty[s]);
       };
@@ -444,25 +653,121 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const uint32_t v_addr = smem_u32(smem + kVOff + s * kTileBytes);
         if (j + 1 < nt) issue_qk(j + 1);
         mbar_wait(&v_full[s], (uint32_t)((j / kStages) & 1), abort_flag, p.status, 203u);
-#pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          mbar_wait(&p_ready[2 * h + g], (uint32_t)(j & 1), abort_flag, p.status, 202u);
-          tc_fence_after();
-#pragma unroll
-          for (int ks = 4 * g; ks < 4 * g + 4; ++ks) {
-            // 16 keys per MMA: P columns 8*ks..8*ks+7 (two bf16 per column), V rows 16*ks.. (2048 bytes apart)
-            // V is MN-major: 64 channels contiguous per key row, the second 64 channels one half-tile further
-            const uint64_t v_desc = make_smem_desc(v_addr + ks * 2048, kHalfBytes, 1024, 2);
-            mma_f16_ts(o_tmem, p_tmem + 8 * ks, v_desc, idesc_pv, (j | ks) != 0);
-          }
-          tc_commit(&pv_done[2 * h + g]);
-        }
+        mbar_wait(&p_ready[2 * h], (uint32_t)(j & 1), abort_flag, p.status, 202u);
+        tc_fence_after();
+        issue_products<0, 4>(o_tmem, p_tmem, v_addr, j != 0);
+        tc_commit(&pv_done[2 * h]);
+        mbar_wait(&p_ready[2 * h + 1], (uint32_t)(j & 1), abort_flag, p.status, 202u);
+        tc_fence_after();
+        issue_products<4, 8>(o_tmem, p_tmem, v_addr, true);
+        tc_commit(&pv_done[2 * h + 1]);
         tc_commit(&v_empty[s]);
+      }
+    }
+  } else if (FUSED && warp >= 12) {
+    if constexpr (FUSED) {
+      // ------------------------------------------------------------------ NVFP4 decode (warps 12..15)
+      // Thread i builds key row i of every tile: first the K stage (the MMAs need it first), then the V stage.
+      setmaxnreg_dec<104>();
+      const int nd = min(nt, p.first_tiles - j0);          // tiles of this CTA that hold cached keys; none where <= 0
+      const int i = (int)threadIdx.x - 384;               // key row of the tile this thread builds; also its table entry
+      const int H = p.heads;
+      const int T = tab.block_tokens;
+      const int n_cached = tab.n_cached, Lk = (int)p.Lk;      // the host keeps the window below 2^31 keys
+      uint8_t* tabs = smem + kTabOff;                       // slot * 4096 + (K: 0, V: 2048) + entry * 16
+      // (block, token) of the first key of the tile being fetched, advanced tile by tile (no divisions in the loop)
+      int fb = (int)(((int64_t)j0 * kBK) / T);
+      int ft = (int)((int64_t)j0 * kBK - (int64_t)fb * T);
+      int fkey = j0 * kBK;
+      // where key row i of the next tile lives, and its scale bytes (global loads, consumed one tile later)
+      auto fetch = [&](RowInfo& r) {
+        const int key = fkey + i;
+        if (key >= n_cached) {
+          r.where = key - n_cached;
+          r.kind = key < Lk ? 1 : 2;
+        } else {
+          const bool second = ft + i >= T;                  // the row lies in the next cache block: second staged code tile
+          const int b = second ? fb + 1 : fb;
+          const int tok = second ? ft + i - T : ft + i;
+          r.kind = 0;
+          r.where = (second ? 128 + tok : i) | ((b % kTabSlots) << 8);
+          const int row = tok * H + head;                   // row of the block: token-major, head-minor
+          const int sf_off = (row >> 7) * 1024 + (row & 31) * 16 + ((row & 127) >> 5) * 4;   // scale columns 0..3; 4..7 are 512 bytes on
+          r.ksf[0] = ld_global(reinterpret_cast<const uint32_t*>(tab.k_sf[b] + sf_off));
+          r.ksf[1] = ld_global(reinterpret_cast<const uint32_t*>(tab.k_sf[b] + sf_off + 512));
+          r.vsf[0] = ld_global(reinterpret_cast<const uint32_t*>(tab.v_sf[b] + sf_off));
+          r.vsf[1] = ld_global(reinterpret_cast<const uint32_t*>(tab.v_sf[b] + sf_off + 512));
+        }
+        fkey += kBK;
+        ft += kBK;
+        if (ft >= T) { ft -= T; ++fb; }
+      };
+      // one of K / V of a tile: expand the staged codes (or copy the current chunk's rows) into stage `st`
+      auto build = [&](const RowInfo& row, int kv, uint32_t sf0, uint32_t sf1, uint8_t* st, uint64_t* codes_full, uint64_t* full,
+                       uint32_t ph) {
+        // the stage is free and its code tiles have landed (the producer waited for the stage before it loaded them)
+        mbar_wait(codes_full, ph, abort_flag, p.status, 400u + kv);
+        uint32_t w[16];
+        if (row.kind == 0) {
+          // 64-byte rows, 16-byte chunks XOR-swizzled with bits 1-2 of the row index (TMA's 64-byte swizzle)
+          const int cr = row.where & 0xFF;
+          const uint8_t* src = st + kCodeOff + cr * 64;
+          const int sw = (cr >> 1) & 3;
+  #pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const uint4 v4 = *reinterpret_cast<const uint4*>(src + ((c ^ sw) << 4));
+            w[4 * c] = v4.x; w[4 * c + 1] = v4.y; w[4 * c + 2] = v4.z; w[4 * c + 3] = v4.w;
+          }
+        }
+        // Both barriers are executed by all 128 threads outside any divergent branch (a tile that mixes cache rows and
+        // current-chunk rows splits a warp between the branches above and below; bar.sync needs converged warps).
+        __syncwarp();
+        asm volatile("bar.sync 1, 128;" ::: "memory");      // every thread holds its codes: the stage's tail may be overwritten
+        if (row.kind == 0) {
+          decode_row(w, sf0, sf1, tabs + (row.where >> 8) * 4096 + kv * 2048, st, i);
+        } else {
+          const uint16_t* src = nullptr;
+          if (row.kind == 1) src = (kv ? tab.v_cur + (int64_t)row.where * tab.ldv : tab.k_cur + (int64_t)row.where * tab.ldk) + (int64_t)head * kD;
+          copy_row(src, st, i);
+        }
+        fence_proxy_async();
+        __syncwarp();
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (i == 0) mbar_arrive(full);
+      };
+      // decode tables exist for cache blocks up to `built`; (lb, lt) = (block, token) of the last key of the current tile
+      int built = fb - 1;
+      int lb = (int)(((int64_t)j0 * kBK + kBK - 1) / T);
+      int lt = (int)((int64_t)j0 * kBK + kBK - 1 - (int64_t)lb * T);
+      const int last_block = n_cached > 0 ? (n_cached - 1) / T : 0;
+      RowInfo nxt;
+      nxt.kind = 2;
+      if (nd > 0) fetch(nxt);
+      for (int j = 0; j < nd; ++j) {
+        const int s = j % kStages;
+        const uint32_t ph = (uint32_t)((j / kStages) & 1);
+        const RowInfo row = nxt;
+        if (j + 1 < nd) fetch(nxt);                         // in flight while this tile is decoded
+        const int b_hi = lb < last_block ? lb : last_block;
+        lt += kBK;
+        if (lt >= T) { lt -= T; ++lb; }
+        if (b_hi > built) {               // the same for all 128 threads; the first barrier of `build` publishes the tables
+          for (int b = built + 1; b <= b_hi; ++b) {
+            uint8_t* tb = tabs + (b % kTabSlots) * 4096;
+            *reinterpret_cast<uint4*>(tb + i * 16) = decode_table_entry((uint32_t)i, __fmul_rn(ld_global(tab.k_amax[b]), tab.inv_denom));
+            *reinterpret_cast<uint4*>(tb + 2048 + i * 16) = decode_table_entry((uint32_t)i, __fmul_rn(ld_global(tab.v_amax[b]), tab.inv_denom));
+          }
+          built = b_hi;
+        }
+  #pragma unroll 1
+        for (int kv = 0; kv < 2; ++kv)                      // K, then V: one copy of the build code
+          build(row, kv, kv ? row.vsf[0] : row.ksf[0], kv ? row.vsf[1] : row.ksf[1], smem + (kv ? kVOff : kKOff) + s * kTileBytes,
+                kv ? &vc_full[s] : &kc_full[s], kv ? &v_full[s] : &k_full[s], ph);
       }
     }
   } else if (warp >= 4) {
     // ------------------------------------------------------------------ softmax + epilogue
-    setmaxnreg_inc<208>();
+    setmaxnreg_inc<FUSED ? 176 : 208>();
     const int q = warp & 3;
     const int half = warp >= 8 ? 1 : 0;
     const uint32_t lane_base = (uint32_t)(q * 32) << 16;
@@ -470,23 +775,41 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     if (half < n_half) {
     float m = -INFINITY;          // exponent offset of the row (raw score units): the row maximum, updated lazily
     float l[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};        // running sum of exp: four packed accumulators
-    const uint32_t s_tmem = tmem_base + lane_base + kSCol;
-    const uint32_t p_tmem = tmem_base + lane_base + kPCol + 64 * half;
+    const uint32_t s_tmem = tmem_base + lane_base + s_col<FUSED>(half);
+    const uint32_t p_tmem = tmem_base + lane_base + p_col<FUSED>(half);
     const uint32_t o_tmem = tmem_base + lane_base + kOCol + 128 * half;
 #pragma unroll 1
     for (int j = 0; j < nt; ++j) {
       const int valid = (int)min((int64_t)kBK, p.Lk - (int64_t)(j0 + j) * kBK);
       mbar_wait(&s_full[half], (uint32_t)(j & 1), abort_flag, p.status, 300u);
       tc_fence_after();
-      uint32_t sr[4][32];
+      // FUSED: 64 scores at a time in rolled loops, read for the maximum and again for the exponentials
+      constexpr int kGroups = FUSED ? 2 : 4, kParts = 4 / kGroups;
+      uint32_t sr[kGroups][32];
+      auto load_scores = [&](int part) {
 #pragma unroll
-      for (int g = 0; g < 4; ++g) tmem_ld32(s_tmem + 32 * g, sr[g]);
-      tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&s_free[half]);       // the other half's scores may take the buffer
-      if (valid < kBK) mask_scores(sr, valid);
-      const float mt = row_max(sr);
+        for (int g = 0; g < kGroups; ++g) tmem_ld32(s_tmem + 32 * (kGroups * part + g), sr[g]);
+        tmem_ld_wait();
+        if (valid < kBK) mask_scores(sr, valid - 32 * kGroups * part);
+      };
+      float mt;
+      if constexpr (FUSED) {
+        mt = -INFINITY;
+#pragma unroll 1
+        for (int part = 0; part < kParts; ++part) {
+          load_scores(part);
+          mt = fmax2(mt, row_max(sr));
+        }
+      } else {
+#pragma unroll
+        for (int g = 0; g < 4; ++g) tmem_ld32(s_tmem + 32 * g, sr[g]);
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_free[half]);       // the other half's scores may take the buffer
+        if (valid < kBK) mask_scores(sr, valid);
+        mt = row_max(sr);
+      }
       // lazy rescale: keep the old offset unless this tile's maximum exceeds it by more than 2^8
       const bool grow = !((mt - m) * c <= 8.f);       // also true for the first tile (m = -inf) and for a NaN
       if (__any_sync(0xFFFFFFFFu, grow)) {
@@ -507,21 +830,26 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // A NaN or +inf score makes the row NaN, as inf - inf does in a softmax: NaN here reaches every exponential of the
       // special-function unit, and with them the row sum.
       const float nmc = __fmaf_rn(-m, c, m - m);
+#pragma unroll 1
+      for (int part = 0; part < kParts; ++part) {
+        if constexpr (FUSED) load_scores(part);
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        uint32_t pk[16];
-        exp_group(sr[g], g, c, nmc, l, pk);
-        // the previous tile's products with this P group must have finished
-        if ((g & 1) == 0 && j > 0) {
-          mbar_wait(&pv_done[2 * half + (g >> 1)], (uint32_t)((j - 1) & 1), abort_flag, p.status, 303u);
-          tc_fence_after();
-        }
-        tmem_st16(p_tmem + 16 * g, pk);
-        if (g & 1) {
-          tmem_st_wait();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&p_ready[2 * half + (g >> 1)]);
+        for (int gg = 0; gg < kGroups; ++gg) {
+          const int g = kGroups * part + gg;
+          uint32_t pk[16];
+          exp_group(sr[gg], gg, c, nmc, l, pk);
+          // the previous tile's products with this P group must have finished (FUSED: they have, S of this tile was issued behind them)
+          if (!FUSED && (g & 1) == 0 && j > 0) {
+            mbar_wait(&pv_done[2 * half + (g >> 1)], (uint32_t)((j - 1) & 1), abort_flag, p.status, 303u);
+            tc_fence_after();
+          }
+          tmem_st16(p_tmem + 16 * g, pk);
+          if (FUSED ? g == 3 : (g & 1)) {
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&p_ready[2 * half + (g >> 1)]);
+          }
         }
       }
     }
@@ -665,17 +993,48 @@ int64_t align256(int64_t n) { return (n + 255) / 256 * 256; }
 // bf16 keys and values of the cached tokens, filled up to whole key tiles with rows of the current chunk
 int64_t window_bytes(int64_t cached, int heads) { return 2 * align256((cached + kBK - 1) / kBK * kBK * heads * kD * 2); }
 
+template <bool FUSED>
 int launch_tiles(dim3 grid, cudaStream_t stream, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmK2,
-                 const CUtensorMap& tmV2, const CUtensorMap& tmO, const AttnParams& p) {
+                 const CUtensorMap& tmV2, const CUtensorMap& tmO, const AttnParams& p, const KvTable<FUSED>& tab) {
+  constexpr uint32_t smem = FUSED ? kSmemBytesFused : kSmemBytes;
   static bool attr_set[64] = {};
   int dev = 0;
   LLNV_CUDA(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    LLNV_CUDA(cudaFuncSetAttribute(attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
+    LLNV_CUDA(cudaFuncSetAttribute(attention_kernel<FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr_set[dev] = true;
   }
-  launch_k(attention_kernel, grid, kThreads, kSmemBytes, stream, tmQ, tmK, tmV, tmK2, tmV2, tmO, p);
+  launch_k(attention_kernel<FUSED>, grid, FUSED ? kThreadsFused : kThreads, smem, stream, tmQ, tmK, tmV, tmK2, tmV2, tmO, p, tab);
   return launch_status("attention_kernel");
+}
+
+// The launch that decodes win's cache blocks in its load stage.
+int launch_fused(dim3 grid, cudaStream_t stream, const CUtensorMap& tmQ, const CUtensorMap& tmK2, const CUtensorMap& tmV2, const CUtensorMap& tmO,
+                 AttnParams p, const CachedWindow& win, const void* k_cur, const void* v_cur, int64_t ldk, int64_t ldv) {
+  LLNV_REQUIRE(p.Lk < INT_MAX - kBK, "llnv_attention_nvfp4kv: a window of %lld keys is too long", (long long)p.Lk);
+  KvTable<true> tab;
+  for (int b = 0; b < win.num_blocks; ++b) {
+    tab.k_sf[b] = (const uint8_t*)win.k_sf[b];
+    tab.k_amax[b] = win.k_amax[b];
+    tab.v_sf[b] = (const uint8_t*)win.v_sf[b];
+    tab.v_amax[b] = win.v_amax[b];
+    // byte matrix [tokens, heads * 64], box 128 tokens x 64 bytes, 64-byte swizzle
+    const uint64_t cols = (uint64_t)p.heads * 64;
+    int rc = cached_tensor_map(&tab.k_codes[b], 0, win.k_codes[b], (uint64_t)win.block_tokens, cols, cols, 128, 64, 2);
+    if (rc == LLNV_OK) rc = cached_tensor_map(&tab.v_codes[b], 0, win.v_codes[b], (uint64_t)win.block_tokens, cols, cols, 128, 64, 2);
+    if (rc != LLNV_OK) return rc;
+  }
+  tab.n_cached = (int)win.tokens();
+  tab.block_tokens = win.block_tokens;
+  tab.inv_denom = (float)(1.0 / (double)win.denom);
+  tab.k_cur = (const uint16_t*)k_cur;
+  tab.v_cur = (const uint16_t*)v_cur;
+  tab.ldk = ldk;
+  tab.ldv = ldv;
+  // what the last tile of the cached part holds of the current chunk is not loaded again
+  p.first_tiles = (tab.n_cached + kBK - 1) / kBK;
+  p.second_row = p.first_tiles * kBK - tab.n_cached;
+  return launch_tiles<true>(grid, stream, tmQ, tmK2, tmV2, tmK2, tmV2, tmO, p, tab);
 }
 
 // Shared host side of the two entry points.  win == nullptr: k / v are the whole window (bf16).  Otherwise the window is win's
@@ -743,37 +1102,31 @@ int attention_launch(const void* q, int64_t Lq, int64_t ldq, const void* k, cons
   tmK = tmK2;
   tmV = tmV2;
 
-  void* own_window = nullptr;
-  if (n_cached > 0) {
-    // the cached part as bf16: behind the partial results in the workspace, or in stream-ordered memory of this call where the
-    // caller's workspace is smaller
-    const int64_t at = align256(zdim > 1 ? split_bytes : 0), bytes = window_bytes(n_cached, heads);
-    uint8_t* kw = (uint8_t*)workspace + at;
-    if (!workspace || ((uintptr_t)workspace & 15) != 0 || workspace_bytes < at + bytes) {
-      LLNV_CUDA(cudaMallocAsync(&own_window, (size_t)bytes, stream));
-      kw = (uint8_t*)own_window;
+  // the cached part as bf16: behind the partial results in the workspace
+  const int64_t at = align256(zdim > 1 ? split_bytes : 0), bytes = window_bytes(n_cached, heads);
+  if (n_cached > 0 && (!workspace || ((uintptr_t)workspace & 15) != 0 || workspace_bytes < at + bytes)) {
+    rc = launch_fused(grid, stream, tmQ, tmK2, tmV2, tmO, p, *win, k, v, ldk, ldv);
+  } else {
+    if (n_cached > 0) {
+      uint8_t* kw = (uint8_t*)workspace + at;
+      uint8_t* vw = kw + bytes / 2;
+      const int64_t first_tiles = (n_cached + kBK - 1) / kBK, rows = first_tiles * kBK;
+      const int64_t pad = rows - n_cached < L_cur ? rows - n_cached : L_cur;
+      rc = kv_window_dequant(win->k_codes, win->k_sf, win->k_amax, win->v_codes, win->v_sf, win->v_amax, win->num_blocks, heads,
+                             win->block_tokens, win->denom, k, v, ldk, ldv, (int)pad, kw, vw, stream);
+      if (rc == LLNV_OK) rc = cached_tensor_map(&tmK, 1, kw, (uint64_t)(n_cached + pad), (uint64_t)C, (uint64_t)C, 128, 64, 3);
+      if (rc == LLNV_OK) rc = cached_tensor_map(&tmV, 1, vw, (uint64_t)(n_cached + pad), (uint64_t)C, (uint64_t)C, 128, 64, 3);
+      p.first_tiles = (int)first_tiles;
+      p.second_row = (int)pad;
     }
-    uint8_t* vw = kw + bytes / 2;
-    const int64_t first_tiles = (n_cached + kBK - 1) / kBK, rows = first_tiles * kBK;
-    const int64_t pad = rows - n_cached < L_cur ? rows - n_cached : L_cur;
-    rc = kv_window_dequant(win->k_codes, win->k_sf, win->k_amax, win->v_codes, win->v_sf, win->v_amax, win->num_blocks, heads,
-                           win->block_tokens, win->denom, k, v, ldk, ldv, (int)pad, kw, vw, stream);
-    if (rc == LLNV_OK) rc = cached_tensor_map(&tmK, 1, kw, (uint64_t)(n_cached + pad), (uint64_t)C, (uint64_t)C, 128, 64, 3);
-    if (rc == LLNV_OK) rc = cached_tensor_map(&tmV, 1, vw, (uint64_t)(n_cached + pad), (uint64_t)C, (uint64_t)C, 128, 64, 3);
-    p.first_tiles = (int)first_tiles;
-    p.second_row = (int)pad;
+    if (rc == LLNV_OK) rc = launch_tiles<false>(grid, stream, tmQ, tmK, tmV, tmK2, tmV2, tmO, p, {});
   }
-  if (rc == LLNV_OK) rc = launch_tiles(grid, stream, tmQ, tmK, tmV, tmK2, tmV2, tmO, p);
   if (rc == LLNV_OK && zdim > 1) {
     const int first_item = tail_cut > 0 ? p.tail_first : 0;
     const int64_t blocks = ((int64_t)q_tiles * heads - first_item) * (kBQ / 8);
     launch_k(attention_combine_kernel, (unsigned)blocks, 256, 0, stream, p.part_o, p.part_ml, zdim, Lq, heads, p.scale_log2, (uint16_t*)out, ldo,
              out_amax, first_item, q_tiles);
     rc = launch_status("attention_combine_kernel");
-  }
-  if (own_window) {
-    const cudaError_t e = cudaFreeAsync(own_window, stream);
-    if (rc == LLNV_OK && e != cudaSuccess) return cuda_fail(e, "cudaFreeAsync");
   }
   return rc;
 }

@@ -262,7 +262,7 @@ SPLIT_TAIL = -1          # LLNV_ATTN_SPLIT_TAIL: cut the tiles of the last parti
 
 
 def attention_workspace_bytes(lq, lk, heads, key_splits=None):
-    """Bytes of workspace ``attention_bf16`` / ``attention_nvfp4kv`` use for this shape (0 when the call is not split);
+    """Bytes of workspace ``attention_bf16`` uses, and ``attention_nvfp4kv`` needs, for this shape (0 when the call is not split);
     ``key_splits`` None = what the library proposes for the current device."""
     lib = _lib.lib()
     if key_splits is None:
@@ -292,11 +292,14 @@ def attention_bf16(q, k, v, heads, scale=None, out=None, key_splits=None, out_am
 def attention_nvfp4kv(q, k_blocks, v_blocks, block_tokens, k_cur, v_cur, heads, scale=None, out=None, key_splits=None,
                       out_amax=None, e2m1_max=6.0, e4m3_max=256.0, workspace=None):
     """Chunk attention over [cached NVFP4 blocks ... | current chunk (bf16)] (``llnv_attention_nvfp4kv``): the cached part is
-    expanded to bf16 in the workspace and attended from there, the current chunk is read in place.  ``k_blocks`` / ``v_blocks``: cache blocks oldest first, each with
-    ``values`` (uint8 [rows_padded, 64]), ``scale_factors`` and ``amax`` (a ``QuantizedTensor`` of
-    ``block_tokens * heads`` rows of 128 channels, token-major / head-minor).  ``k_cur`` / ``v_cur``: bf16
+    expanded to bf16 in the workspace and attended from there, the current chunk is read in place.  ``k_blocks`` / ``v_blocks``:
+    cache blocks oldest first, each with ``values`` (uint8 [rows_padded, 64]), ``scale_factors`` and ``amax`` (a
+    ``QuantizedTensor`` of ``block_tokens * heads`` rows of 128 channels, token-major / head-minor).  ``k_cur`` / ``v_cur``: bf16
     [L_cur, heads*128] (or None when the window is the cache alone).  Result: bf16 [Lq, heads*128], equal bit
-    for bit to dequantizing the blocks into a window and calling ``attention_bf16`` on it."""
+    for bit to dequantizing the blocks into a window and calling ``attention_bf16`` on it.
+    ``workspace``: a uint8 tensor of ``attention_nvfp4kv_workspace_bytes``, allocated per call when omitted; one that holds the
+    partial results of a split call alone (``attention_workspace_bytes``, any size for an unsplit one) has the blocks decoded inside
+    the attention kernel, which is slower on long windows and takes no memory for them."""
     return _lib.native().attention_nvfp4kv(q, _seq(k_blocks), _seq(v_blocks), int(block_tokens), k_cur, v_cur, heads, scale, out,
                                            _opt_int(key_splits), out_amax, e2m1_max, e4m3_max, workspace)
 

@@ -413,3 +413,43 @@ def test_merge_of_many_splits(splits):
     out = ops.attention_bf16(q, k, v, heads, key_splits=splits, out_amax=amax[1]).float()
     assert float((out - ref).norm() / ref.norm()) < 4e-3
     assert float(amax[1]) == float(out.abs().max()) and float(amax[0]) == float(ref.abs().max())
+
+
+@pytest.mark.parametrize("lq,heads,T,blocks,l_cur,splits", [
+    (270, 2, 128, 3, 0, 1),           # blocks of exactly one key tile, no current chunk
+    (130, 1, 129, 16, 129, 1),        # as many blocks as a call takes, each boundary at another key of its tile
+    (300, 3, 200, 4, 1, 3),           # one key of the current chunk, in the last cached tile
+    (100, 2, 880, 2, 880, 5),         # one query half only, a split that begins behind the cache
+    (2640, 14, 528, 4, 528, None),    # 154 items: the last wave of them is cut
+])
+def test_nvfp4kv_without_room_for_the_window(lq, heads, T, blocks, l_cur, splits):
+    """A workspace for the partial results alone: no expanded window, no allocation, one launch fewer, also in a captured graph; the result
+    is that of the call with room, bit for bit."""
+    g = torch.Generator(device="cuda").manual_seed(lq)
+    kq, vq = _cache_blocks(blocks, T, heads, g), _cache_blocks(blocks, T, heads, g)
+    q = torch.randn(lq, heads * 128, generator=g, device="cuda").bfloat16()
+    cur = [torch.randn(l_cur, heads * 128, generator=g, device="cuda").bfloat16() if l_cur else None for _ in range(2)]
+    lib = _lib.lib()
+    if splits is None:
+        splits = lib.llnv_attention_key_splits(lq, blocks * T + l_cur, heads)
+        assert splits == ops.SPLIT_TAIL
+    amax = [torch.zeros(1, device="cuda") for _ in range(2)]
+    before = lib.llnv_launch_count()
+    ref = ops.attention_nvfp4kv(q, kq, vq, T, *cur, heads, key_splits=splits, out_amax=amax[0])
+    with_room = lib.llnv_launch_count() - before
+    ws = torch.full((max(16, ops.attention_workspace_bytes(lq, blocks * T + l_cur, heads, key_splits=splits)),), 0xFF, dtype=torch.uint8, device="cuda")
+    out = torch.zeros_like(ref)
+    call = lambda: ops.attention_nvfp4kv(q, kq, vq, T, *cur, heads, key_splits=splits, workspace=ws, out=out, out_amax=amax[1])
+    before = lib.llnv_launch_count()
+    call()
+    assert lib.llnv_launch_count() - before == with_room - 1
+    assert torch.equal(out, ref) and torch.equal(*amax)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call()
+    out.zero_()
+    for _ in range(2):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert lib.llnv_check_status(None) == 0, lib.llnv_last_error()
+    assert torch.equal(out, ref)
