@@ -42,29 +42,48 @@ using namespace quant;
 // Largest magnitude among every `stride`-th group of kAmaxLoads x 256 16-byte vectors of x (M rows of K elements, ldx apart),
 // starting with group `first`, as the bits of the 16-bit type: bf16 and fp16 magnitudes both order as integers.  Called by the
 // 256 threads of a CTA; thread 0 has the result.  A thread keeps eight loads in flight: with one load and one division of the
-// index per step the pass over 2640 x 14336 took 24.6 us (3.1 TB/s), now 14.3 us.  ROWS: rows are further apart than their length, the index is
-// divided into row and column.
+// index per step the pass over 2640 x 14336 took 24.6 us (3.1 TB/s), now 14.3 us.
+// Behind the end a thread reads its vector 0 again, which no maximum minds: conditional loads were issued one by one.
+// ROWS: rows are further apart than their length.  A step of the CTA is then a power of two of vectors of as many rows as that leaves
+// threads for, so that which rows and vectors a step covers is the same for all threads and no thread divides.
 constexpr int kAmaxLoads = 8;
 template <bool ROWS>
 __device__ __forceinline__ uint32_t cta_amax_bits(const uint16_t* x, int64_t M, int64_t K, int64_t ldx, unsigned first,
                                                   unsigned stride) {
   const int64_t vec_per_row = K >> 3;
-  const int64_t total = M * vec_per_row;
+  const uint4* xv = reinterpret_cast<const uint4*>(x);
   uint32_t m = 0;   // two 15-bit magnitudes, compared as unsigned 16-bit lanes
-  for (int64_t i0 = (int64_t)first * (kAmaxLoads * 256) + threadIdx.x; i0 < total; i0 += (int64_t)stride * (kAmaxLoads * 256)) {
-    uint4 v[kAmaxLoads];
-#pragma unroll
-    for (int j = 0; j < kAmaxLoads; ++j) {
-      const int64_t i = i0 + j * 256;
-      v[j] = make_uint4(0u, 0u, 0u, 0u);
-      if (i < total) {
-        const int64_t r = ROWS ? i / vec_per_row : 0;
-        v[j] = ld_global(reinterpret_cast<const uint4*>(x + r * ldx) + (i - r * vec_per_row));
-      }
-    }
+  auto take = [&](const uint4 (&v)[kAmaxLoads]) {
 #pragma unroll
     for (int j = 0; j < kAmaxLoads; ++j)
       m = __vmaxu2(m, __vmaxu2(__vmaxu2(v[j].x & 0x7FFF7FFFu, v[j].y & 0x7FFF7FFFu), __vmaxu2(v[j].z & 0x7FFF7FFFu, v[j].w & 0x7FFF7FFFu)));
+  };
+  if (ROWS) {
+    const int log_w = vec_per_row >= 256 ? 8 : 31 - __clz((int)vec_per_row);       // a step: 2^log_w vectors of 256 >> log_w rows
+    const int64_t step_rows = 256 >> log_w, row_step = step_rows * (ldx >> 3);     // (rows are 16-byte aligned)
+    const int64_t row_steps = (M + step_rows - 1) >> (8 - log_w), col_steps = (vec_per_row + (1 << log_w) - 1) >> log_w, steps = row_steps * col_steps;
+    const int64_t my_r = threadIdx.x >> log_w, my_c = threadIdx.x & ((1 << log_w) - 1), my_off = my_r * (ldx >> 3) + my_c;
+    for (int64_t s0 = (int64_t)first * kAmaxLoads; s0 < steps; s0 += (int64_t)stride * kAmaxLoads) {
+      int64_t rs = steps <= 0xFFFFFFFFll ? (uint32_t)s0 / (uint32_t)col_steps : s0 / col_steps, cs = s0 - rs * col_steps;
+      uint4 v[kAmaxLoads];
+#pragma unroll
+      for (int j = 0; j < kAmaxLoads; ++j) {
+        const int64_t off = rs * row_step + (cs << log_w) + my_off;
+        v[j] = ld_global(xv + ((rs * step_rows + my_r < M) & ((cs << log_w) + my_c < vec_per_row) ? off : 0));
+        const bool wrap = ++cs == col_steps;
+        cs = wrap ? 0 : cs;
+        rs = wrap ? rs + 1 : rs;
+      }
+      take(v);
+    }
+  } else {
+    const int64_t total = M * vec_per_row;
+    for (int64_t i0 = (int64_t)first * (kAmaxLoads * 256) + threadIdx.x; i0 < total; i0 += (int64_t)stride * (kAmaxLoads * 256)) {
+      uint4 v[kAmaxLoads];
+#pragma unroll
+      for (int j = 0; j < kAmaxLoads; ++j) v[j] = ld_global(xv + (i0 + j * 256 < total ? i0 + j * 256 : 0));
+      take(v);
+    }
   }
   uint32_t mm = max(m & 0xFFFFu, m >> 16);
 #pragma unroll
@@ -427,9 +446,15 @@ __global__ void div_const_selftest_kernel(uint32_t first, uint64_t count, unsign
   if (bad) atomicAdd(mismatches, bad);
 }
 
-// Up to here every CTA of the quantizer reads the whole tensor for its amax (kPlainAmax).  us for the call with the separate memset
-// and amax launches / with this: 24576 elements 11.4 / 6.2, 52224 11.3 / 7.4, 129024 12.3 / 10.3.
-constexpr int64_t kOwnAmaxElements = 131072;
+// Whether every CTA of the quantizer takes the amax of the whole tensor itself (kPlainAmax), instead of a memset and an amax launch in
+// front of it: a CTA's pass grows with the tensor, and what the CTAs read together with their number too.  Device us of the call with
+// the separate launches / this: 17 x 3072 8.2 / 5.1, 42 x 3072 8.2 / 7.0, 1 x 32768 8.7 / 7.6, 16 x 8192 8.2 / 6.8, 4 x 14336 8.2 / 8.6
+// (two launches fewer); beyond: 9 x 14336 8.2 / 12.6, 1 x 131072 14.4 / 21.6.  Rows apart: 17 x 3072 8.2 / 7.2, 128 x 512 8.3 / 7.2,
+// 1 x 14336 8.2 / 7.3; beyond: 42 x 3072 8.3 / 11.8, 4 x 14336 8.2 / 13.2.
+bool own_amax_pays(int64_t M, int64_t K, int64_t ctas, bool contiguous) {
+  const int64_t n = M * K;
+  return contiguous ? n <= 131072 && ctas * n <= ((int64_t)1 << 23) : n <= 65536 && ctas * n <= ((int64_t)1 << 21);
+}
 
 template <bool F16>
 int launch_amax(const void* x, int64_t M, int64_t K, int64_t ldx, float* amax, cudaStream_t stream) {
@@ -549,14 +574,13 @@ extern "C" int llnv_quantize_nvfp4_ex(const void* x, int64_t M, int64_t K, int64
     if (!amax_given) LLNV_CUDA(cudaMemsetAsync(amax, 0, sizeof(float), stream));
     return LLNV_OK;
   }
-  // Of a small tensor every CTA of the quantizer takes the amax itself, instead of a memset and an amax launch in front of it
-  const bool own_amax = !amax_given && M * K <= kOwnAmaxElements;
+  const int64_t mp = (M + 127) / 128 * 128, grid_x = (K + 127) / 128;
+  const bool own_amax = !amax_given && own_amax_pays(M, K, grid_x * (mp / 128), ldx == Ks);
   if (!amax_given && !own_amax) {
     int rc = llnv_amax_bf16(x, M * shards, Ks, ldx, amax, stream_);
     if (rc != LLNV_OK) return rc;
   }
-  const int64_t mp = (M + 127) / 128 * 128;
-  dim3 grid((unsigned)((K + 127) / 128), (unsigned)(mp / 128));
+  dim3 grid((unsigned)grid_x, (unsigned)(mp / 128));
   LLNV_REQUIRE(mp / 128 <= 65535, "llnv_quantize_nvfp4: too many rows (%lld)", (long long)M);
   Prologue pr = {};
   if (shards > 1) {

@@ -7,7 +7,7 @@ import pytest
 import torch
 
 import longlive_b200 as L
-from longlive_b200 import ops
+from longlive_b200 import _lib, ops
 from oracle import nvfp4_oracle as O
 from tests import util
 
@@ -267,3 +267,37 @@ def test_quantize_amax_forms_agree(m, k):
         q = ops.quantize_nvfp4(t, 3)
         assert float(q[2].item()) == float(amax) == float(ops.amax_bf16(t).item())
         assert np.array_equal(util.u8(q[1]), sf) and np.array_equal(q[0].cpu().numpy(), codes)
+
+
+@pytest.mark.parametrize("m,k,apart,own", [
+    (16, 8192, False, True), (1, 32768, False, True), (1, 32832, False, False), (5, 14336, False, True), (6, 14336, False, False), (1, 131072, False, False),
+    (21, 3072, True, True), (22, 3072, True, False), (128, 512, True, True), (1, 16384, True, True), (1, 16448, True, False), (3, 192, True, True),
+])
+def test_amax_inside_the_quantizer_where_its_reads_are_few(m, k, apart, own):
+    """The quantizer's CTAs take the amax themselves where they read little for it together, on both sides of the rule's lines."""
+    x = util.config_activation(m, k, seed=k)
+    codes, sf, amax = O.quantize_nvfp4(x.float().numpy(), "mse")
+    t = torch.full((m, k + 16), 1e4, dtype=torch.bfloat16, device="cuda")[:, :k].copy_(x) if apart else x.cuda()
+    q = ops.quantize_nvfp4(t, 3)
+    before = _lib.lib().llnv_launch_count()
+    q = ops.quantize_nvfp4(t, 3)
+    assert _lib.lib().llnv_launch_count() - before == (1 if own else 2)
+    assert float(q[2].item()) == float(amax)
+    assert np.array_equal(util.u8(q[1]), sf) and np.array_equal(q[0].cpu().numpy(), codes)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("m,k", [(1, 64), (2, 2048), (255, 24 * 64), (257, 320), (4000, 64), (300, 37 * 64), (33, 2112)])
+def test_amax_of_rows_apart_finds_the_largest_anywhere(m, k, dtype):
+    """The largest value at the first, the last and some other places, with larger ones between the rows: row lengths that are and are not a
+    power of two of vectors, one step and many."""
+    g = torch.Generator().manual_seed(m + k)
+    wide = torch.full((m, k + 8), 500.0, dtype=dtype, device="cuda")
+    t = wide[:, :k]
+    cfg = L.QuantizationConfig(scale_rule="static_6")
+    for place in [0, m * k - 1, k - 1, (m - 1) * k, *torch.randint(0, m * k, (6,), generator=g).tolist()]:
+        t.fill_(0.5)
+        t[place // k, place % k] = -3.0
+        assert float(L.quantize_to_fp4(t, cfg).amax.item()) == 3.0, place
+        if dtype == torch.bfloat16:
+            assert float(ops.amax_bf16(t).item()) == 3.0, place
