@@ -301,3 +301,26 @@ def test_amax_of_rows_apart_finds_the_largest_anywhere(m, k, dtype):
         assert float(L.quantize_to_fp4(t, cfg).amax.item()) == 3.0, place
         if dtype == torch.bfloat16:
             assert float(ops.amax_bf16(t).item()) == 3.0, place
+
+
+@pytest.mark.parametrize("rule", ["mse", "mae"])
+def test_quantize_blocks_of_few_values_match_oracle(rule):
+    """Blocks of one, two and three values with every bf16 mantissa and both signs, and of sixteen equal ones: the two candidates often
+    stand for the same values, which the quantizer sees without their errors."""
+    g = torch.Generator().manual_seed(11)
+    mant = (1 + torch.arange(128) / 128).repeat(2) * torch.tensor([1.0] * 128 + [-1.0] * 128)
+    rows = [mant.repeat_interleave(16)]                                       # all equal
+    for others in ((), (2 / 3,), (1 / 6, 1 / 3), (-1 / 12, 1.0), (0.25, 0.04)):
+        b = torch.zeros(256, 16)
+        pos = torch.randint(0, 13, (256,), generator=g)
+        b[torch.arange(256), pos] = mant
+        for i, f in enumerate(others):
+            b[torch.arange(256), pos + 1 + i] = mant * f
+        rows.append(b.reshape(-1))
+    x = torch.stack([r * 2.0 ** e for r in rows for e in (-6, -1, 0)]).bfloat16()
+    x = torch.cat([x, x[:1] * 1.37])                                          # another tensor maximum
+    for t in (x[:-1], x):
+        codes, sf, amax = O.quantize_nvfp4(t.float().numpy(), rule)
+        q = L.quantize_to_fp4(t.cuda(), L.QuantizationConfig(scale_rule=rule))
+        assert float(q.amax.item()) == float(amax)
+        assert np.array_equal(util.u8(q.scale_factors), sf) and np.array_equal(q.values.cpu().numpy(), codes)
