@@ -9,6 +9,7 @@
 
 #include <cstdarg>
 #include <cstdio>
+#include <utility>
 
 #include "../../include/llnvfp4.h"
 
@@ -69,8 +70,9 @@ bool pdl_enabled();                    // llnv_set_pdl(0) / environment LLNV_PDL
 void count_launch();                   // llnv_launch_count(): kernels launched by the library since it was loaded
 bool amax_accumulate(int which);       // llnv_set_amax_accumulate: bit 1 attention + LN quantizers, bit 2 grouped GEMM + RoPE
 
+// `overlap`: whether the launch may overlap its predecessor at all (see the caller that says no).
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+inline cudaError_t launch_k_if(bool overlap, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -80,9 +82,13 @@ inline cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() && !capturing(stream) ? 1 : 0;
+  cfg.numAttrs = overlap && pdl_enabled() && !capturing(stream) ? 1 : 0;
   count_launch();
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  return launch_k_if(true, kernel, grid, block, smem, stream, std::forward<Args>(args)...);
 }
 
 // ---- group maximum over NVLink peer memory, for kernels that consume a tensor amax --------------

@@ -196,3 +196,22 @@ def test_a_blocked_launch_leaves_other_threads_running(op):
     ticker.join()
     assert longest > 0.1, "the launch queue never filled"
     assert max(gaps) < longest / 2
+
+
+@pytest.mark.parametrize("m", [100, 1000, 4000])
+def test_fp16_quantizer_overlapped_or_not(pdl, m):
+    """The fp16 quantizer, whose launch overlaps its predecessor below and above a device full of CTAs but not between, reads what that
+    predecessor wrote."""
+    g = torch.Generator(device="cuda").manual_seed(m)
+    w, xs = torch.eye(256, dtype=torch.bfloat16, device="cuda").repeat(12, 1), torch.randn(3, m, 256, generator=g, device="cuda").bfloat16()
+    runs = []
+    for on in (0, 1):
+        pdl(on)
+        x, keep = torch.empty(m, 3072, dtype=torch.float16, device="cuda"), []
+        for i in range(6):
+            x.copy_(ops.linear_bf16(xs[i % 3], w))
+            ops.quantize_nvfp4(xs[(i + 1) % 3], 3)
+            keep.append([_bits(t) for t in ops.quantize_nvfp4(x, 3)])
+        torch.cuda.synchronize()
+        runs.append(keep)
+    _same(*runs)
