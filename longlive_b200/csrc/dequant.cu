@@ -59,24 +59,17 @@ __device__ __forceinline__ void store16<float>(float* out, const float (&v)[16])
     reinterpret_cast<float4*>(out)[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
 }
 
-template <typename T>
-__device__ __forceinline__ void store8(T* out, const float (&v)[8]);
-template <>
-__device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16* out, const float (&v)[8]) {
+// 16 bytes of output: 8 values of 16 bits or 4 of 32
+__device__ __forceinline__ void store_vec(__nv_bfloat16* out, const float (&v)[8]) {
   *reinterpret_cast<uint4*>(out) = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
 }
-template <>
-__device__ __forceinline__ void store8<__half>(__half* out, const float (&v)[8]) {
+__device__ __forceinline__ void store_vec(__half* out, const float (&v)[8]) {
   __half2 h[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) h[i] = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
   *reinterpret_cast<uint4*>(out) = *reinterpret_cast<uint4*>(&h[0]);
 }
-template <>
-__device__ __forceinline__ void store8<float>(float* out, const float (&v)[8]) {
-  reinterpret_cast<float4*>(out)[0] = make_float4(v[0], v[1], v[2], v[3]);
-  reinterpret_cast<float4*>(out)[1] = make_float4(v[4], v[5], v[6], v[7]);
-}
+__device__ __forceinline__ void store_vec(float* out, const float (&v)[4]) { *reinterpret_cast<float4*>(out) = make_float4(v[0], v[1], v[2], v[3]); }
 
 // decode 8 packed bytes (16 codes) and scale them
 template <int ROUNDING>
@@ -124,13 +117,13 @@ __global__ void __launch_bounds__(256) dequant_matrix_kernel(const uint8_t* code
 
 // KV cache: block b holds `rows` logical rows of 128 columns.
 //
-// Bound by HBM writes (2 bytes out for 9/16 in).  A lane decodes one code word = 8 values = one 16-byte store, so a warp's
-// store covers 512 contiguous bytes (with 16 values a thread the two halves of a sector came from two instructions and cost
-// two partial writes); a CTA of 256 threads covers 16 rows a step and takes kKvSteps steps whose loads are issued together.
-// 4 blocks of 2640 x 24 rows (8 with keys and values): see the entry points.
-constexpr int kKvSteps = 4;
-constexpr int kKvRows = 16 * kKvSteps;
-template <typename T, int ROUNDING>
+// Bound by HBM writes (2 bytes out for 9/16 in).  A lane decodes the values of one 16-byte store, so a warp's store covers
+// 512 contiguous bytes (with 16 values a thread the two halves of a sector came from two instructions and cost
+// two partial writes); a CTA of 256 threads covers 4 KB of output a step and takes STEPS steps whose loads are issued together: four, or
+// one where that leaves SMs without a CTA (660 x 3 rows with a division per value 7.3 us with four steps, 3.1 with one).
+// us for 4 blocks of 2640 x 24 rows in L2: bf16 13.0, fp32 24.9 (37.0 with 8 values a lane, two stores 32 bytes apart), with a division per
+// value 56 and 58.
+template <typename T, int ROUNDING, int STEPS>
 __global__ void __launch_bounds__(256) dequant_kv_kernel(const __grid_constant__ BlockTable tab, int num_blocks, int64_t rows, float denom,
                                                          const __grid_constant__ RowCopies copies) {
   pdl_begin();
@@ -146,36 +139,38 @@ __global__ void __launch_bounds__(256) dequant_kv_kernel(const __grid_constant__
     }
     return;
   }
-  const int c = threadIdx.x & 15;                            // code word of the row: columns 8c .. 8c + 7
-  const int64_t r0 = (int64_t)blockIdx.x * kKvRows + (threadIdx.x >> 4);
-  const uint32_t* codes = reinterpret_cast<const uint32_t*>(tab.codes[b]);
+  constexpr int kVals = 16 / sizeof(T), kLanes = 128 / kVals, kStepRows = 256 / kLanes;
+  const int c = threadIdx.x % kLanes;                        // columns kVals * c .. kVals * c + kVals - 1
+  const int64_t r0 = (int64_t)blockIdx.x * (kStepRows * STEPS) + threadIdx.x / kLanes;
+  const uint8_t* codes = tab.codes[b];
   const uint8_t* sf = tab.sf[b];
-  uint32_t w[kKvSteps], sb[kKvSteps];
+  uint32_t w[STEPS], sb[STEPS];
 #pragma unroll
-  for (int k = 0; k < kKvSteps; ++k) {
-    const int64_t r = r0 + 16 * k;
+  for (int k = 0; k < STEPS; ++k) {
+    const int64_t r = r0 + kStepRows * k;
     w[k] = sb[k] = 0u;
     if (r < rows) {
-      w[k] = ld_global(codes + r * 16 + c);
-      sb[k] = ld_global(sf + sf_offset(r, c >> 1, 8));
+      if (kVals == 8) w[k] = ld_global(reinterpret_cast<const uint32_t*>(codes) + r * 16 + c);
+      else w[k] = ld_global(reinterpret_cast<const uint16_t*>(codes) + r * 32 + c);
+      sb[k] = ld_global(sf + sf_offset(r, c * kVals / 16, 8));
     }
   }
   const float amax = ld_global(tab.amax[b]);
   const float g = global_scale(ROUNDING, amax, denom);
   T* out = (T*)tab.out[b];
 #pragma unroll
-  for (int k = 0; k < kKvSteps; ++k) {
-    const int64_t r = r0 + 16 * k;
+  for (int k = 0; k < STEPS; ++k) {
+    const int64_t r = r0 + kStepRows * k;
     if (r >= rows) continue;
     const float s = e4m3_to_float(sb[k]);
-    float v[8];
+    float v[kVals];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < kVals / 2; ++i) {
       const __half2_raw h2 = __nv_cvt_fp4x2_to_halfraw2((__nv_fp4x2_storage_t)(uint8_t)(w[k] >> (8 * i)), __NV_E2M1);
       v[2 * i] = deq_scale<ROUNDING>(__fmul_rn(__half2float(__ushort_as_half(h2.x)), s), amax, g, denom);
       v[2 * i + 1] = deq_scale<ROUNDING>(__fmul_rn(__half2float(__ushort_as_half(h2.y)), s), amax, g, denom);
     }
-    store8<T>(out + r * 128 + c * 8, v);
+    store_vec(out + r * 128 + c * kVals, v);
   }
 }
 
@@ -196,19 +191,26 @@ int launch_matrix(const uint8_t* codes, const uint8_t* sf, const float* amax, in
   return launch_status("dequant_matrix_kernel");
 }
 
-template <typename T>
-int launch_kv(const BlockTable& tab, int n, int64_t rows, float denom, int rounding, const RowCopies& copies, cudaStream_t stream) {
-  const int extra = copies.rows > 0 ? 2 : 0;
-  if (rows * n == 0 && extra == 0) return LLNV_OK;
-  const int64_t gx = (rows + kKvRows - 1) / kKvRows;
+template <typename T, int STEPS>
+int launch_kv_steps(const BlockTable& tab, int n, int64_t rows, float denom, int rounding, const RowCopies& copies, cudaStream_t stream) {
+  constexpr int kCtaRows = 2 * 16 / sizeof(T) * STEPS;
+  const int64_t gx = (rows + kCtaRows - 1) / kCtaRows;
   LLNV_REQUIRE(gx < ((int64_t)1 << 31), "llnv_kv_dequant: too many rows (%lld)", (long long)rows);
-  const dim3 grid((unsigned)gx, (unsigned)(n + extra));
+  const dim3 grid((unsigned)gx, (unsigned)(n + (copies.rows > 0 ? 2 : 0)));
   switch (rounding) {
-    case LLNV_DEQ_FUSED: launch_k(dequant_kv_kernel<T, LLNV_DEQ_FUSED>, grid, 256, 0, stream, tab, n, rows, denom, copies); break;
-    case LLNV_DEQ_PYTORCH: launch_k(dequant_kv_kernel<T, LLNV_DEQ_PYTORCH>, grid, 256, 0, stream, tab, n, rows, denom, copies); break;
-    default: launch_k(dequant_kv_kernel<T, LLNV_DEQ_TRITON>, grid, 256, 0, stream, tab, n, rows, denom, copies); break;
+    case LLNV_DEQ_FUSED: launch_k(dequant_kv_kernel<T, LLNV_DEQ_FUSED, STEPS>, grid, 256, 0, stream, tab, n, rows, denom, copies); break;
+    case LLNV_DEQ_PYTORCH: launch_k(dequant_kv_kernel<T, LLNV_DEQ_PYTORCH, STEPS>, grid, 256, 0, stream, tab, n, rows, denom, copies); break;
+    default: launch_k(dequant_kv_kernel<T, LLNV_DEQ_TRITON, STEPS>, grid, 256, 0, stream, tab, n, rows, denom, copies); break;
   }
   return launch_status("dequant_kv_kernel");
+}
+
+template <typename T>
+int launch_kv(const BlockTable& tab, int n, int64_t rows, float denom, int rounding, const RowCopies& copies, cudaStream_t stream) {
+  if (rows * n == 0 && copies.rows == 0) return LLNV_OK;
+  const int64_t ctas = (rows + 63) / 64 * n;                 // of four steps of 16 rows
+  if (ctas < 2 * (int64_t)sm_count()) return launch_kv_steps<T, 1>(tab, n, rows, denom, rounding, copies, stream);
+  return launch_kv_steps<T, 4>(tab, n, rows, denom, rounding, copies, stream);
 }
 
 }  // namespace

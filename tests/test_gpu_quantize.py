@@ -324,3 +324,19 @@ def test_quantize_blocks_of_few_values_match_oracle(rule):
         q = L.quantize_to_fp4(t.cuda(), L.QuantizationConfig(scale_rule=rule))
         assert float(q.amax.item()) == float(amax)
         assert np.array_equal(util.u8(q.scale_factors), sf) and np.array_equal(q.values.cpu().numpy(), codes)
+
+
+@pytest.mark.parametrize("rounding", [ops.DEQ_FUSED, ops.DEQ_PYTORCH, ops.DEQ_TRITON])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("tokens,heads,blocks", [(1, 1, 1), (31, 1, 2), (33, 3, 1), (129, 1, 33), (801, 8, 3)])
+def test_kv_dequant_equals_the_matrix_form(tokens, heads, blocks, dtype, rounding):
+    """One and four steps a thread, rows that end inside a step, 8 and 4 values a lane, more blocks than one launch takes: the same bits as
+    the matrix kernel gives block by block."""
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    rows = tokens * heads
+    qs = [L.quantize_to_fp4((torch.randn(rows, 128, generator=g, device="cuda") * (1 + i)).bfloat16()) for i in range(blocks)]
+    out = ops.kv_dequant([q.values for q in qs], [q.scale_factors for q in qs], [q.amax for q in qs], heads, tokens, dtype, 6, 256, rounding)
+    assert out.shape == (1, blocks * tokens, heads, 128)
+    for i, q in enumerate(qs):
+        ref = ops.dequantize_nvfp4(q.values, q.scale_factors, q.amax, rows, 128, 128, dtype, 6, 256, rounding)
+        assert torch.equal(out[0, i * tokens:(i + 1) * tokens].reshape(rows, 128), ref), i
